@@ -70,6 +70,12 @@ __device__ __forceinline__ float3 xnormalize(float3 v) {
 }
 
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
+// 32 bytes in one load (256-bit global loads, sm_100): p 32-byte aligned.
+__device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
 __device__ __forceinline__ int fbits_i(float f) { return __float_as_int(f); }
 __device__ __forceinline__ uint32_t fbits_u(float f) { return __float_as_uint(f); }
 
