@@ -212,15 +212,13 @@ struct SceneHit {
 template <bool kCurves>
 __device__ __forceinline__ SceneHit finish_closest(const Traversal& T, float tmax) {
     SceneHit h;
-    h.t = T.tri >= 0 ? T.closest : tmax;
-    h.u = T.u;
-    h.v = T.v;
-    h.prim = T.tri >= 0 ? uint32_t(T.tri) : kMiss;
+    h.prim = T.prim;
+    h.t = h.prim != kMiss ? T.closest : tmax;
+    h.u = h.prim != kMiss ? T.u : 0.f;
+    h.v = h.prim != kMiss ? T.v : 0.f;
     h.tang = f3(0.f, 0.f, 0.f);
     h.tseg = 0.f;
-    if (kCurves && T.seg >= 0) {
-        h.t = T.closest;
-        h.prim = 0x80000000u | uint32_t(T.seg);
+    if (kCurves && h.prim != kMiss && (h.prim & 0x80000000u)) {
         h.tang = T.tang;
         h.tseg = T.tseg;
         h.u = 0.f;
@@ -229,10 +227,7 @@ __device__ __forceinline__ SceneHit finish_closest(const Traversal& T, float tma
     return h;
 }
 
-template <bool kCurves>
-__device__ __forceinline__ bool finish_any(const Traversal& T) {
-    return T.tri >= 0 || (kCurves && T.seg >= 0);
-}
+__device__ __forceinline__ bool finish_any(const Traversal& T) { return T.prim != kMiss; }
 
 __device__ __forceinline__ void warp_add_work(unsigned long long* work, const Counters& cnt) {
     unsigned long long a = cnt.nodes, b = cnt.prims, c = cnt.segs, e = cnt.cnodes;
@@ -261,40 +256,37 @@ __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uin
     if constexpr (kPersist) {
         persistent_traverse<kAny, kCount, kCurves, kMotion, kPark>(S, n, fetch, err, cnt, load, done);
     } else {
-        uint2 stack[kMaxStack4];
+        uint2 local[kFrame + kMaxStack4 + 1];
+        uint2* const stack = local + kFrame;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             Ray ray;
             uint32_t root, segRoot;
             load(i, ray, root, segRoot);
             Traversal T;
-            trav_init(T, ray, root);
+            trav_init<kCurves, kMotion>(T, ray, root, segRoot, i, stack);
             while (true) {
-                while (true) {
-                    while (!T.exhausted) {
-                        if (!(T.cur & 0x80000000u)) {
-                            node_step<kAny, kCount, kCurves>(T, S, stack, err, cnt);
-                        } else if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, cnt)) {
-                            T.exhausted = true;
-                        } else if (!trav_pop<kAny>(T, stack)) {
-                            T.exhausted = true;
-                        }
+                do {
+                    while (T.cur != kEmptyChild) {
+                        if (int(T.cur) >= 0) node_step<kAny, kCount, kCurves>(T, S, stack, err, cnt);
+                        else if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, stack, cnt)) T.cur = kEmptyChild;
+                        else trav_pop<kAny>(T, stack);
                     }
-                    if (stage_done<kAny, kCurves>(T, ray.d, segRoot)) break;
-                }
+                } while (!stage_done<kAny, kCurves>(T, stack));
+                trav_finish<kCurves>(T, stack);
                 Ray next;
                 if (!trace_again(done, i, T, next)) break;
-                trav_init(T, next, root);
+                trav_init<kCurves, kMotion>(T, next, root, segRoot, i, stack);
             }
         }
     }
 }
 
-// Persistent triangle kernels fit 5 blocks per SM (48 registers, a few spills
-// to L1; on the throughput frame 451 ms against 467 ms at 4 blocks and 64
-// registers, and 520 ms at 6 blocks and 40); the motion variants (object-ray
-// state) keep 4 and 64 registers; with the curve stage they take 3 (80
-// registers with spills to L1: the ribbon test's state; the hair frame
-// 1280x720x32 measured 1699 ms against 1813 ms at 2 blocks and 128).
+// Persistent triangle kernels fit 5 blocks per SM at 48 registers without
+// spills (1920x1080x64 throughput frame: 290.2 ms; 293.8 at 56 registers and
+// 36 warps per SM, 292.2 at 40 and 48 warps); the motion variants (object-ray
+// state) keep 4 and 64 registers; with the curve stage they take 3 and 80 (the
+// ribbon test's state; 1280x720x8 hair frame 260.0 ms against 285.1 at 4
+// blocks and 64 registers).
 #define ANA_TRAVERSAL_BOUNDS \
     __launch_bounds__(kPersistBlock, kPersist ? (kCurves ? 3 : (kMotion ? 4 : kPersistMinBlocks)) : 1)
 
@@ -729,7 +721,7 @@ __global__ void ANA_TRAVERSAL_BOUNDS k_shadow(const __grid_constant__ Params p) 
         },
         [&](uint32_t i, const Traversal& T) {
             float4 o = p.q.sh_o[i], c = p.q.sh_c[i];
-            const bool occluded = finish_any<kCurves>(T);
+            const bool occluded = finish_any(T);
             if (!occluded) add_L(p, __float_as_uint(o.w), f3(c));
             if constexpr (kAdj) p.a.sh_vis[i] = occluded ? 0u : 1u;
         });
@@ -763,7 +755,7 @@ __global__ void ANA_TRAVERSAL_BOUNDS k_mis(const __grid_constant__ Params p) {
             float3 Li;
             int mi = -1;
             if (kAny) {
-                Li = finish_any<kCurves>(T) ? f3(0.f, 0.f, 0.f) : scene_env(S, R, rd);
+                Li = finish_any(T) ? f3(0.f, 0.f, 0.f) : scene_env(S, R, rd);
             } else {
                 SceneHit h = finish_closest<kCurves>(T, 1e10f);
                 if (h.prim == kMiss) {
@@ -1062,7 +1054,7 @@ __global__ void ANA_TRAVERSAL_BOUNDS k_trace_batch(const __grid_constant__ DevSc
     run_traversal<kAny, false, kPersist, kCurves, kMotion>(S, n, fetch, err, nullptr, load, [&](uint32_t i, const Traversal& T) {
         ana_hit h{0, -1, -1, -1, 0.f, 0.f, 0.f, 0.f};
         if (kAny) {
-            h.hit = finish_any<kCurves>(T) ? 1 : 0;
+            h.hit = finish_any(T) ? 1 : 0;
         } else {
             const float tmax = reinterpret_cast<const float4*>(rays + 8 * size_t(i))[1].w;
             SceneHit sh = finish_closest<kCurves>(T, tmax);

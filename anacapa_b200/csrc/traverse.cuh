@@ -26,9 +26,9 @@ struct Ray {
 // safe(v) = |v| > 1e-9 ? v : 1e-9 (the sign of tiny components is dropped),
 // and the triangle test rebuilds dir = 1/invDir.
 struct TriRay {
-    float3 o, inv, dir;
+    float3 o, inv;
     float tmin, tmax;
-    bool nx, ny, nz;
+    uint32_t neg;  // bit i: direction component i is negative
 };
 
 __device__ __forceinline__ float safe_comp(float v) { return fabsf(v) > 1e-9f ? v : 1e-9f; }
@@ -37,35 +37,52 @@ __device__ __forceinline__ TriRay make_tri_ray(const Ray& r) {
     TriRay q;
     q.o = r.o;
     q.inv = f3(xdiv(1.f, safe_comp(r.d.x)), xdiv(1.f, safe_comp(r.d.y)), xdiv(1.f, safe_comp(r.d.z)));
-    q.dir = f3(xdiv(1.f, q.inv.x), xdiv(1.f, q.inv.y), xdiv(1.f, q.inv.z));
     q.tmin = r.tmin;
     q.tmax = r.tmax;
-    q.nx = r.d.x < 0.f;
-    q.ny = r.d.y < 0.f;
-    q.nz = r.d.z < 0.f;
+    q.neg = (r.d.x < 0.f ? 1u : 0u) | (r.d.y < 0.f ? 2u : 0u) | (r.d.z < 0.f ? 4u : 0u);
     return q;
 }
+__device__ __forceinline__ float3 tri_dir(const TriRay& q) {
+    return f3(xdiv(1.f, q.inv.x), xdiv(1.f, q.inv.y), xdiv(1.f, q.inv.z));
+}
 
-// Slab test of one child box. Returns true and tNear when the box is entered
-// before `cull` (the current closest hit) and its interval is not empty.
-__device__ __forceinline__ bool box_hit(const TriRay& r, float lox, float hix, float loy, float hiy,
-                                        float loz, float hiz, float cull, float& tnear) {
-    float nx = r.nx ? hix : lox, fx = r.nx ? lox : hix;
-    float ny = r.ny ? hiy : loy, fy = r.ny ? loy : hiy;
-    float nz = r.nz ? hiz : loz, fz = r.nz ? loz : hiz;
-    float t0x = xmul(xsub(nx, r.o.x), r.inv.x), t1x = xmul(xsub(fx, r.o.x), r.inv.x);
-    float t0y = xmul(xsub(ny, r.o.y), r.inv.y), t1y = xmul(xsub(fy, r.o.y), r.inv.y);
-    float t0z = xmul(xsub(nz, r.o.z), r.inv.z), t1z = xmul(xsub(fz, r.o.z), r.inv.z);
-    float tmn = fmaxf(fmaxf(fmaxf(r.tmin, t0x), t0y), t0z);
-    float tmx = fminf(fminf(fminf(r.tmax, t1x), t1y), t1z);
-    tnear = tmn;
-    return tmx > tmn && tmn <= cull;
+// (p - o) * inv of two boxes' planes of one axis, each operation rounded on
+// its own (packed single precision: two boxes per instruction).
+__device__ __forceinline__ float2 plane_pair(float p, float q, float o, float inv) {
+    float2 r;
+    asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n mov.b64 c, {%5, %5};\n"
+        " add.rn.f32x2 a, a, b;\n mul.rn.f32x2 a, a, c;\n mov.b64 {%0, %1}, a;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(p), "f"(q), "f"(-o), "f"(inv));
+    return r;
+}
+
+// Slab distances of four child boxes (lo / hi: the boxes' planes by axis): the
+// entries (from the ray's tmin) and the exits (from its tmax). A box's near
+// plane is its high one where the direction is negative.
+__device__ __forceinline__ void box_slabs(const TriRay& r, const float (&lo)[3][4], const float (&hi)[3][4],
+                                          float (&tn)[4], float (&tf)[4]) {
+    const float o[3] = {r.o.x, r.o.y, r.o.z}, inv[3] = {r.inv.x, r.inv.y, r.inv.z};
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+        float2 n[3], f[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const bool neg = r.neg & (1u << i);
+            n[i] = plane_pair(neg ? hi[i][k] : lo[i][k], neg ? hi[i][k + 1] : lo[i][k + 1], o[i], inv[i]);
+            f[i] = plane_pair(neg ? lo[i][k] : hi[i][k], neg ? lo[i][k + 1] : hi[i][k + 1], o[i], inv[i]);
+        }
+        tn[k] = fmaxf(fmaxf(fmaxf(r.tmin, n[0].x), n[1].x), n[2].x);
+        tn[k + 1] = fmaxf(fmaxf(fmaxf(r.tmin, n[0].y), n[1].y), n[2].y);
+        tf[k] = fminf(fminf(fminf(r.tmax, f[0].x), f[1].x), f[2].x);
+        tf[k + 1] = fminf(fminf(fminf(r.tmax, f[0].y), f[1].y), f[2].y);
+    }
 }
 
 // Moller-Trumbore, BVHBackend::intersectTriangle.
-__device__ __forceinline__ bool tri_hit(const TriRay& r, float3 v0, float3 e1, float3 e2, float tmax,
+__device__ __forceinline__ bool tri_hit(const TriRay& r, float3 dir, float3 v0, float3 e1, float3 e2, float tmax,
                                         float& t, float& u, float& v) {
-    float3 h = xcross(r.dir, e2);
+    float3 h = xcross(dir, e2);
     float a = xdot(e1, h);
     if (fabsf(a) < 1e-9f) return false;
     float f = xdiv(1.f, a);
@@ -73,7 +90,7 @@ __device__ __forceinline__ bool tri_hit(const TriRay& r, float3 v0, float3 e1, f
     u = xmul(f, xdot(s, h));
     if (u < 0.f || u > 1.f) return false;
     float3 q = xcross(s, e1);
-    v = xmul(f, xdot(r.dir, q));
+    v = xmul(f, xdot(dir, q));
     if (v < 0.f || xadd(u, v) > 1.f) return false;
     t = xmul(f, xdot(e2, q));
     return t >= r.tmin && t <= tmax;
@@ -101,8 +118,8 @@ struct Counters {
 //      next queue entries together (one warp-aggregated atomicAdd on the
 //      stage's fetch counter);
 //   2. interior phase: lanes descend interior nodes until they reach a
-//      leaf; the phase ends when every lane has a leaf to test (or nothing
-//      left), when no lane can take another interior step, or when at most
+//      leaf; the phase ends when no lane can take another interior step, when
+//      every lane has parked a leaf or has nothing left, or when at most
 //      kLeafPhaseLanes (any hit: kLeafPhaseLanesAny) lanes still descend
 //      while others wait with a leaf, so lanes stay converged on the
 //      node-test code. Any-hit queries can be speculative (kPark; Aila and
@@ -115,7 +132,7 @@ struct Counters {
 //      and MIS kernels too, and only the curve shadow kernels and the
 //      occlusion queries of ana_trace_batch park);
 //   3. leaf phase: the parked leaf's (else the current leaf's) triangles.
-// A lane whose stack is exhausted (or, for occlusion, that found a blocker)
+// A lane whose stack is used up (or, for occlusion, that found a blocker)
 // reports its ray and picks up a new one at the next refill, so finished rays
 // do not idle the warp until its slowest ray completes. Box and triangle
 // tests are the same functions as above, so results are identical.
@@ -154,60 +171,104 @@ constexpr int kRefillLanesCurves = 4;
 constexpr int kRefillLanesCurvesAny = 4;
 
 struct Traversal {
-    TriRay r;
-    float closest, u, v;
-    int32_t tri;
+    TriRay r;        // curve stage: r.inv is the exact 1/d
+    float closest;
+    uint32_t prim;   // closest hit so far: leaf-order triangle, 0x80000000 | segment, or kNoPrim
     uint32_t cur;
     int sp;
-    bool exhausted;
     // curve stage (scenes with curves): the triangle BVH is traversed first,
     // then the curve BVH from the triangle hit distance (CurveBrute::trace)
-    uint32_t stage;  // 0 triangles, 1 curves
-    int32_t seg;     // leaf-order segment of the closest ribbon hit, -1 if none
-    float tseg;
+    bool curve;      // the curve BVH is being traversed
+    bool flat;       // a direction component is below CurveBrute::aabbHit's 1e-9
+    // filled from the frame when the ray is reported
+    float u, v, tseg;
     float3 tang;
-    float3 cd, fx, fy, cinv;  // exact direction, ray-space frame x/y, 1/d
-    float time;               // ray time: object rays of motion-blurred triangles
 };
+constexpr uint32_t kNoPrim = 0xFFFFFFFFu;
+
+// A lane's local memory: kFrame slots, then the traversal stack. The slots
+// below stack[0] hold what the node steps never read, so that the registers
+// hold the interior loop's own values: with all of the ray's state in
+// registers the compiler spilled some of those instead and reloaded them at
+// every node (1920x1080x64 throughput frame: extend stage 108.0 -> 103.2 ms;
+// 1280x720x8 hair frame 264.5 -> 260.0 ms).
+//   -1 (u, v) of the closest triangle hit     -2, -3.x direction of the
+//   -3.y queue entry                             primitive tests
+//   -4, -5.x exact direction, -5.y curve root (triangle stage); from the curve
+//   stage on -4 .. -6 the ray frame's x and y axes
+//   -7, -8 (tangent, strand parameter) of the closest ribbon hit
+//   -9.x ray time, -9.y, -10 exact direction (motion)
+constexpr int kFrame = 10;
+
+__device__ __forceinline__ uint2 pair(float a, float b) { return make_uint2(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ float lo(uint2 p) { return __uint_as_float(p.x); }
+__device__ __forceinline__ float hi(uint2 p) { return __uint_as_float(p.y); }
+__device__ __forceinline__ float3 frame_dir(const uint2* stack) {
+    const uint2 a = stack[-2];
+    return f3(lo(a), hi(a), lo(stack[-3]));
+}
 
 // Starts a traversal at a scene's root (kNoRoot: the scene has no triangles).
 // Closest hit keeps the nearest accepted triangle; ties (t == closest) go to
 // the later-tested triangle, as `t <= r.tMax` does in the reference; any hit
 // (kAny) stops at the first accepted triangle (BVHBackend::occluded,
 // BVHBackend.cpp:409-444).
-__device__ __forceinline__ void trav_init(Traversal& T, const Ray& ray, uint32_t root) {
+template <bool kCurves, bool kMotion>
+__device__ __forceinline__ void trav_init(Traversal& T, const Ray& ray, uint32_t root, uint32_t segRoot, uint32_t idx,
+                                          uint2* stack) {
     T.r = make_tri_ray(ray);
-    T.cd = ray.d;  // read by the motion test (and reset by curve_begin)
-    T.time = ray.time;
     T.closest = ray.tmax;
-    T.u = T.v = 0.f;
-    T.tri = -1;
+    T.prim = kNoPrim;
     T.cur = root;
-    T.sp = 0;
-    T.exhausted = root == kNoRoot;
-    T.stage = 0;
-    T.seg = -1;
+    T.sp = 1;
+    stack[0] = make_uint2(kEmptyChild, __float_as_uint(-INFINITY));
+    T.curve = false;
+    T.flat = false;
+    const float3 d = tri_dir(T.r);
+    stack[-2] = pair(d.x, d.y);
+    stack[-3] = make_uint2(__float_as_uint(d.z), idx);
+    if (kCurves) {
+        stack[-4] = pair(ray.d.x, ray.d.y);
+        stack[-5] = make_uint2(__float_as_uint(ray.d.z), segRoot);
+    }
+    if (kMotion) {
+        stack[-9] = pair(ray.time, ray.d.x);
+        stack[-10] = pair(ray.d.y, ray.d.z);
+    }
 }
 
+// The closest hit's parameters, for the report.
+template <bool kCurves>
+__device__ __forceinline__ void trav_finish(Traversal& T, const uint2* stack) {
+    const uint2 a = stack[-1];
+    T.u = lo(a);
+    T.v = hi(a);
+    if (kCurves) {
+        const uint2 b = stack[-7], c = stack[-8];
+        T.tang = f3(lo(b), hi(b), lo(c));
+        T.tseg = hi(c);
+    }
+}
+
+// Takes the next stack entry; stack[0] is an entry that is never culled and
+// ends the traversal (cur = kEmptyChild), so a pop tests no stack depth and a
+// lane's state is its current entry alone: an interior node (bit 31 clear), a
+// leaf, or kEmptyChild for nothing left or no ray (1280x720x8 hair frame 260.0
+// -> 250.0 ms, 1279x719x16 glass frame 11.55 -> 11.34 ms against flags).
 // Traversal stack entry (thread-local memory): x = node or leaf entry, y = the
 // entry distance's bits (closest hit; any hit writes x only). One 64-bit
 // access per push and pop instead of two 32-bit ones: the throughput frame's
 // extend stage 116.4 -> 115.7 ms, the 1920x1080x64 hair frame 4549 -> 4505 ms.
 template <bool kAny = false>
-__device__ __forceinline__ bool trav_pop(Traversal& T, const uint2* stack) {
+__device__ __forceinline__ void trav_pop(Traversal& T, const uint2* stack) {
     if (kAny) {  // an any-hit query ends at its first hit: nothing on the stack is culled
-        if (T.sp == 0) return false;
         T.cur = stack[--T.sp].x;
-        return true;
+        return;
     }
-    while (T.sp > 0) {
-        --T.sp;
-        const uint2 e = stack[T.sp];
-        if (__uint_as_float(e.y) > T.closest) continue;
-        T.cur = e.x;
-        return true;
-    }
-    return false;
+    uint2 e;
+    do e = stack[--T.sp];
+    while (__uint_as_float(e.y) > T.closest);
+    T.cur = e.x;
 }
 
 // Interior step: one 128-byte node fetch and four child-box tests. The
@@ -244,7 +305,7 @@ __device__ __forceinline__ void cswap(float& ka, uint32_t& va, float& kb, uint32
 __device__ __forceinline__ void enter_near_first(Traversal& T, float (&key)[4], uint32_t (&ref)[4], uint2* stack, uint32_t* err) {
     const int n = int(key[0] < INFINITY) + int(key[1] < INFINITY) + int(key[2] < INFINITY) + int(key[3] < INFINITY);
     if (n == 0) {
-        if (!trav_pop(T, stack)) T.exhausted = true;
+        trav_pop(T, stack);
         return;
     }
     if (n == 1) {  // one child entered: it becomes the current node
@@ -258,9 +319,9 @@ __device__ __forceinline__ void enter_near_first(Traversal& T, float (&key)[4], 
         uint32_t ra = h0 ? ref[0] : h1 ? ref[1] : ref[2];
         float kb = g3 ? key[3] : g2 ? key[2] : key[1];
         uint32_t rb = g3 ? ref[3] : g2 ? ref[2] : ref[1];
-        if (T.sp + 1 > int(kMaxStack4)) {
+        if (T.sp > int(kMaxStack4)) {
             atomicOr(err, 1u);
-            T.exhausted = true;
+            T.cur = kEmptyChild;
             return;
         }
         cswap(ka, ra, kb, rb);
@@ -275,9 +336,9 @@ __device__ __forceinline__ void enter_near_first(Traversal& T, float (&key)[4], 
     cswap(key[0], ref[0], key[2], ref[2]);
     cswap(key[1], ref[1], key[3], ref[3]);
     cswap(key[1], ref[1], key[2], ref[2]);
-    if (T.sp + n - 1 > int(kMaxStack4)) {
+    if (T.sp + n - 2 > int(kMaxStack4)) {
         atomicOr(err, 1u);
-        T.exhausted = true;
+        T.cur = kEmptyChild;
         return;
     }
 #pragma unroll
@@ -290,49 +351,155 @@ __device__ __forceinline__ void enter_near_first(Traversal& T, float (&key)[4], 
     T.cur = ref[0];
 }
 
-// A node's boxes and references in four loads. A warp's lanes read different
-// nodes, so every load instruction costs the L1 one tag lookup per active
-// lane; with one 32-byte load per axis instead of two of 16 bytes a node takes
-// four lookups instead of seven (1920x1080x64 throughput frame: extend stage
-// 114.7 -> 109.2 ms, shadow 52.6 -> 48.7, MIS 67.4 -> 64.1).
-__device__ __forceinline__ void load_node(const Bvh4Node* n, float4& lx, float4& hx, float4& ly, float4& hy,
-                                          float4& lz, float4& hz, float4& rf) {
-    const float4* np = reinterpret_cast<const float4*>(n);
+// BVHBackend::makeObjectSpaceRay4: the world ray (origin, exact direction)
+// taken to the object space of motion mesh `mm` at the ray's time.
+__device__ __forceinline__ TriRay object_ray(const DevScene& S, uint32_t mm, const Traversal& T, const uint2* stack,
+                                             float tmax) {
+    M4 o2w, w2o;
+    const uint2 a = stack[-9], b = stack[-10];
+    o2w_at(S, mm, lo(a), o2w);
+    m4_inverse(o2w, w2o);
+    Ray r;
+    r.o = m4_point(w2o, T.r.o);
+    r.d = m4_vector(w2o, f3(hi(a), lo(b), hi(b)));
+    r.tmin = T.r.tmin;
+    r.tmax = tmax;
+    r.time = lo(a);
+    return make_tri_ray(r);
+}
+
+// Tests the triangles of leaf entry `leaf`; true when an any-hit query found
+// its blocker. kMotion: triangles flagged object-space (bit 31 of the index
+// word) meet the ray in their mesh's object space at the ray's time.
+template <bool kAny, bool kCount, bool kMotion = false>
+__device__ __forceinline__ bool leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack, Counters* cnt) {
+    const float3 dir = frame_dir(stack);
+    const uint32_t off = leaf & 0x01FFFFFFu, c = ((leaf >> 25) & 63u) + 1u;
+    // the object ray of the leaf's last motion mesh, reused while the mesh
+    // repeats (the same value the reference recomputes per triangle)
+    uint32_t cachedMM = 0xFFFFFFFFu;
+    TriRay ro;
+    float3 rodir;
+    for (uint32_t i = off; i < off + c; ++i) {
+        const float4* tp = S.tri_isect + 3 * size_t(i);
+        float4 a = ldg4(tp), b = ldg4(tp + 1), e = ldg4(tp + 2);
+        if (kCount) cnt->prims++;
+        float t, u, v;
+        const float tmax = kAny ? T.r.tmax : T.closest;
+        bool h;
+        if (kMotion && (__float_as_uint(a.w) & 0x80000000u)) {
+            const uint32_t mm = __float_as_uint(b.w);
+            if (mm != cachedMM) {
+                ro = object_ray(S, mm, T, stack, tmax);
+                rodir = tri_dir(ro);
+                cachedMM = mm;
+            }
+            h = tri_hit(ro, rodir, f3(a), f3(b), f3(e), tmax, t, u, v);
+        } else {
+            h = tri_hit(T.r, dir, f3(a), f3(b), f3(e), tmax, t, u, v);
+        }
+        if (h) {
+            T.closest = t;
+            T.prim = i;
+            if (kAny) return true;
+            stack[-1] = pair(u, v);
+        }
+    }
+    return false;
+}
+
+// ===========================================================================
+// Curves
+// ===========================================================================
+
+// CurveBrute::aabbHit (CurveBrute.cpp:478-498).
+__device__ __noinline__ float curve_key_flat(float3 ro, float3 rd, float3 inv, float tmin, float maxT,
+                                              const float* box) {
+    float tmn = tmin, tmx = maxT;
+    const float lo[3] = {box[0], box[8], box[16]}, hi[3] = {box[4], box[12], box[20]};
+    const float o[3] = {ro.x, ro.y, ro.z}, d[3] = {rd.x, rd.y, rd.z}, iv[3] = {inv.x, inv.y, inv.z};
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        if (fabsf(d[i]) < 1e-9f) {
+            if (o[i] < lo[i] || o[i] > hi[i]) return INFINITY;
+            continue;
+        }
+        float t0 = xmul(xsub(lo[i], o[i]), iv[i]);
+        float t1 = xmul(xsub(hi[i], o[i]), iv[i]);
+        if (iv[i] < 0.f) {
+            float tt = t0;
+            t0 = t1;
+            t1 = tt;
+        }
+        tmn = fmaxf(tmn, t0);
+        tmx = fminf(tmx, t1);
+        if (tmx < tmn) return INFINITY;
+    }
+    return tmn;
+}
+
+// The four keys of a curve node for a ray with a direction component below
+// 1e-9, whose slab that component does not divide by.
+__device__ __forceinline__ void curve_keys_flat(const Traversal& T, const uint2* stack, const float4* np,
+                                                float (&key)[4]) {
+    const float* f = reinterpret_cast<const float*>(np);
+    const float3 d = frame_dir(stack);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        key[k] = __float_as_uint(f[24 + k]) == kEmptyChild
+                     ? INFINITY
+                     : curve_key_flat(T.r.o, d, T.r.inv, T.r.tmin, T.closest, f + k);
+}
+
+// One node of either BVH: one 128-byte read in four loads (a warp's lanes read
+// different nodes, so every load costs the L1 one tag lookup per active lane;
+// with one 32-byte load per axis instead of two of 16 bytes a node takes four
+// lookups instead of seven: 1920x1080x64 throughput frame, extend stage 114.7
+// -> 109.2 ms, shadow 52.6 -> 48.7, MIS 67.4 -> 64.1). Triangle boxes (BVHBackend::intersectAABB) are
+// entered when tMin..tMax of the slabs is not empty and starts no later than
+// the closest hit; curve boxes (CurveBrute::aabbHit) when the slabs' interval
+// up to the closest hit is not reversed. Both stages share one copy of the
+// loads and slab tests, so lanes in different stages step together; curve boxes
+// tested axis by axis with an early exit took the 1280x720x8 hair frame 297.5
+// ms against 264.5 without branches. The slab tests run packed, two boxes per
+// instruction (glass frame 11.34 -> 11.20 ms, throughput 289.5 -> 288.5 ms).
+template <bool kAny, bool kCount, bool kCurves>
+__device__ __forceinline__ void node_step(Traversal& T, const DevScene& S, uint2* stack, uint32_t* err, Counters* cnt) {
+    const bool curve = kCurves && T.curve;
+    const float4* np = reinterpret_cast<const float4*>((curve ? S.seg_nodes : S.tri_nodes) + T.cur);
+    float4 lx, hx, ly, hy, lz, hz;
     ldg8(np, lx, hx);
     ldg8(np + 2, ly, hy);
     ldg8(np + 4, lz, hz);
-    rf = ldg4(np + 6);
-}
-
-template <bool kAny, bool kCount>
-__device__ __forceinline__ void trav_interior(Traversal& T, const DevScene& S, uint2* stack,
-                                              uint32_t* err, Counters* cnt) {
-    float4 lx, hx, ly, hy, lz, hz, rf;
-    load_node(S.tri_nodes + T.cur, lx, hx, ly, hy, lz, hz, rf);
-    if (kCount) cnt->nodes++;
+    const float4 rf = ldg4(np + 6);
+    if (kCount) {
+        if (curve) cnt->cnodes++;
+        else cnt->nodes++;
+    }
     const float cull = kAny ? T.r.tmax : T.closest;
     float key[4];
     uint32_t ref[4] = {fbits_u(rf.x), fbits_u(rf.y), fbits_u(rf.z), fbits_u(rf.w)};
     {
-        const float l0[4] = {lx.x, lx.y, lx.z, lx.w}, h0[4] = {hx.x, hx.y, hx.z, hx.w};
-        const float l1[4] = {ly.x, ly.y, ly.z, ly.w}, h1[4] = {hy.x, hy.y, hy.z, hy.w};
-        const float l2[4] = {lz.x, lz.y, lz.z, lz.w}, h2[4] = {hz.x, hz.y, hz.z, hz.w};
+        const float blo[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w}, {lz.x, lz.y, lz.z, lz.w}};
+        const float bhi[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w}, {hz.x, hz.y, hz.z, hz.w}};
+        float tn[4], tf[4];
+        box_slabs(T.r, blo, bhi, tn, tf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float tn;
-            const bool h = ref[k] != kEmptyChild && box_hit(T.r, l0[k], h0[k], l1[k], h1[k], l2[k], h2[k], cull, tn);
-            key[k] = h ? tn : INFINITY;
+            const bool in = curve ? !(fminf(tf[k], cull) < tn[k]) : (tf[k] > tn[k] && tn[k] <= cull);
+            key[k] = ref[k] != kEmptyChild && in ? tn[k] : INFINITY;
         }
     }
-    if constexpr (kAny) {  // any hit: children entered in stored order, no distance sort
+    if (kCurves && curve && T.flat) curve_keys_flat(T, stack, np, key);
+    if (kAny && !curve) {  // any hit: children entered in stored order, no distance sort
         const int n = int(key[0] < INFINITY) + int(key[1] < INFINITY) + int(key[2] < INFINITY) + int(key[3] < INFINITY);
         if (n == 0) {
-            if (!trav_pop<kAny>(T, stack)) T.exhausted = true;
+            trav_pop<kAny>(T, stack);
             return;
         }
-        if (T.sp + n - 1 > int(kMaxStack4)) {
+        if (T.sp + n - 2 > int(kMaxStack4)) {
             atomicOr(err, 1u);
-            T.exhausted = true;
+            T.cur = kEmptyChild;
             return;
         }
         uint32_t first = kEmptyChild;
@@ -349,99 +516,6 @@ __device__ __forceinline__ void trav_interior(Traversal& T, const DevScene& S, u
     enter_near_first(T, key, ref, stack, err);
 }
 
-// BVHBackend::makeObjectSpaceRay4: the world ray (origin, exact direction)
-// taken to the object space of motion mesh `mm` at the ray's time.
-__device__ __forceinline__ TriRay object_ray(const DevScene& S, uint32_t mm, const Traversal& T, float tmax) {
-    M4 o2w, w2o;
-    o2w_at(S, mm, T.time, o2w);
-    m4_inverse(o2w, w2o);
-    Ray r;
-    r.o = m4_point(w2o, T.r.o);
-    r.d = m4_vector(w2o, T.cd);
-    r.tmin = T.r.tmin;
-    r.tmax = tmax;
-    r.time = T.time;
-    return make_tri_ray(r);
-}
-
-// Tests the triangles of leaf entry `leaf`; true when an any-hit query found
-// its blocker. kMotion: triangles flagged object-space (bit 31 of the index
-// word) meet the ray in their mesh's object space at the ray's time.
-template <bool kAny, bool kCount, bool kMotion = false>
-__device__ __forceinline__ bool leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, Counters* cnt) {
-    const uint32_t off = leaf & 0x01FFFFFFu, c = ((leaf >> 25) & 63u) + 1u;
-    // the object ray of the leaf's last motion mesh, reused while the mesh
-    // repeats (the same value the reference recomputes per triangle)
-    uint32_t cachedMM = 0xFFFFFFFFu;
-    TriRay ro;
-    for (uint32_t i = off; i < off + c; ++i) {
-        const float4* tp = S.tri_isect + 3 * size_t(i);
-        float4 a = ldg4(tp), b = ldg4(tp + 1), e = ldg4(tp + 2);
-        if (kCount) cnt->prims++;
-        float t, u, v;
-        const float tmax = kAny ? T.r.tmax : T.closest;
-        bool h;
-        if (kMotion && (__float_as_uint(a.w) & 0x80000000u)) {
-            const uint32_t mm = __float_as_uint(b.w);
-            if (mm != cachedMM) {
-                ro = object_ray(S, mm, T, tmax);
-                cachedMM = mm;
-            }
-            h = tri_hit(ro, f3(a), f3(b), f3(e), tmax, t, u, v);
-        } else {
-            h = tri_hit(T.r, f3(a), f3(b), f3(e), tmax, t, u, v);
-        }
-        if (h) {
-            T.closest = t;
-            T.u = u;
-            T.v = v;
-            T.tri = int32_t(i);
-            if (kAny) return true;
-        }
-    }
-    return false;
-}
-
-// Leaf step of the one-thread-per-ray schedule: test the current leaf, then pop.
-template <bool kAny, bool kCount>
-__device__ __forceinline__ void trav_leaf(Traversal& T, const DevScene& S, const uint2* stack, Counters* cnt) {
-    if (leaf_test<kAny, kCount>(T, S, T.cur, cnt)) {
-        T.exhausted = true;
-        return;
-    }
-    if (!trav_pop<kAny>(T, stack)) T.exhausted = true;
-}
-
-// ===========================================================================
-// Curves
-// ===========================================================================
-
-// CurveBrute::aabbHit (CurveBrute.cpp:478-498).
-__device__ __forceinline__ bool curve_box_hit(const Ray& r, float3 inv, float lox, float hix, float loy,
-                                              float hiy, float loz, float hiz, float maxT, float& tnear) {
-    float tmn = r.tmin, tmx = maxT;
-    float lo[3] = {lox, loy, loz}, hi[3] = {hix, hiy, hiz};
-    float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z}, iv[3] = {inv.x, inv.y, inv.z};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        if (fabsf(d[i]) < 1e-9f) {
-            if (o[i] < lo[i] || o[i] > hi[i]) return false;
-            continue;
-        }
-        float t0 = xmul(xsub(lo[i], o[i]), iv[i]);
-        float t1 = xmul(xsub(hi[i], o[i]), iv[i]);
-        if (iv[i] < 0.f) {
-            float tt = t0;
-            t0 = t1;
-            t1 = tt;
-        }
-        tmn = fmaxf(tmn, t0);
-        tmx = fminf(tmx, t1);
-        if (tmx < tmn) return false;
-    }
-    tnear = tmn;
-    return true;
-}
 
 // Ray-space frame of makeRayFrame (CurveBrute.cpp:29-47): z = direction, x/y
 // from buildOrthonormalBasis (Types.h:108-114).
@@ -614,45 +688,30 @@ __device__ __forceinline__ bool ribbon_hit(const RayFrame& fr, float tmin, float
 // Node and leaf steps mirror the triangle ones, so both stages share the
 // converged interior / leaf phases and the stack.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void curve_begin(Traversal& T, float3 d, uint32_t segRoot) {
-    T.stage = 1;
-    T.cd = d;
-    onb_exact(d, T.fx, T.fy);
-    T.cinv = f3(xdiv(1.f, d.x), xdiv(1.f, d.y), xdiv(1.f, d.z));
+__device__ __forceinline__ void curve_begin(Traversal& T, uint2* stack) {
+    const uint2 a = stack[-4], b = stack[-5];
+    const float3 d = f3(lo(a), hi(a), lo(b));
+    const uint32_t segRoot = b.y;
+    float3 fx, fy;
+    onb_exact(d, fx, fy);
+    T.curve = true;
+    T.flat = fabsf(d.x) < 1e-9f || fabsf(d.y) < 1e-9f || fabsf(d.z) < 1e-9f;
+    T.r.inv = f3(xdiv(1.f, d.x), xdiv(1.f, d.y), xdiv(1.f, d.z));
     T.cur = segRoot;
-    T.sp = 0;
-    T.exhausted = segRoot == kNoRoot;
-}
-
-// One curve-BVH node: four child boxes (CurveBrute::aabbHit), entered nearest
-// first for closest and any hit alike (on the hair frame near-first any-hit
-// steps measured faster than the stored order).
-template <bool kCount>
-__device__ __forceinline__ void curve_interior(Traversal& T, const DevScene& S, uint2* stack,
-                                               uint32_t* err, Counters* cnt) {
-    const Ray ray{T.r.o, T.cd, T.r.tmin, T.r.tmax};
-    float4 lx, hx, ly, hy, lz, hz, rf;
-    load_node(S.seg_nodes + T.cur, lx, hx, ly, hy, lz, hz, rf);
-    if (kCount) cnt->cnodes++;
-    float key[4];
-    uint32_t ref[4] = {fbits_u(rf.x), fbits_u(rf.y), fbits_u(rf.z), fbits_u(rf.w)};
-    const float l0[4] = {lx.x, lx.y, lx.z, lx.w}, h0[4] = {hx.x, hx.y, hx.z, hx.w};
-    const float l1[4] = {ly.x, ly.y, ly.z, ly.w}, h1[4] = {hy.x, hy.y, hy.z, hy.w};
-    const float l2[4] = {lz.x, lz.y, lz.z, lz.w}, h2[4] = {hz.x, hz.y, hz.z, hz.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float tn = 0.f;
-        const bool h = ref[k] != kEmptyChild &&
-                       curve_box_hit(ray, T.cinv, l0[k], h0[k], l1[k], h1[k], l2[k], h2[k], T.closest, tn);
-        key[k] = h ? tn : INFINITY;
-    }
-    enter_near_first(T, key, ref, stack, err);
+    T.sp = 1;  // stack[0] still ends the stack
+    stack[-2] = pair(d.x, d.y);
+    stack[-3].x = __float_as_uint(d.z);
+    stack[-4] = pair(fx.x, fx.y);
+    stack[-5] = pair(fx.z, fy.x);
+    stack[-6] = pair(fy.y, fy.z);
 }
 
 // Ribbon tests of one curve leaf; true when an any-hit query found its blocker.
 template <bool kAny, bool kCount>
-__device__ __forceinline__ bool curve_leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, Counters* cnt) {
-    const RayFrame fr{T.r.o, T.fx, T.fy, T.cd};
+__device__ __forceinline__ bool curve_leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack,
+                                                Counters* cnt) {
+    const uint2 p4 = stack[-4], p5 = stack[-5], p6 = stack[-6];
+    const RayFrame fr{T.r.o, f3(lo(p4), hi(p4), lo(p5)), f3(hi(p5), lo(p6), hi(p6)), frame_dir(stack)};
     const uint32_t off = leaf & 0x01FFFFFFu, c = ((leaf >> 25) & 63u) + 1u;
     for (uint32_t i = off; i < off + c; ++i) {
         const float4* sp4 = S.segs + 5 * size_t(i);
@@ -661,35 +720,29 @@ __device__ __forceinline__ bool curve_leaf_test(Traversal& T, const DevScene& S,
         float ts, bt = T.closest;
         float3 tg;
         if (ribbon_hit(fr, T.r.tmin, f3(a), f3(b), f3(e), f3(g), a.w, b.w, e.w, g.w, bt, ts, tg)) {
-            T.seg = int32_t(i);
+            T.prim = 0x80000000u | i;
             T.closest = bt;
-            T.tseg = ts;
-            T.tang = tg;
             if (kAny) return true;
+            stack[-7] = pair(tg.x, tg.y);
+            stack[-8] = pair(tg.z, ts);
         }
     }
     return false;
 }
 
-// Stage dispatch of the node and leaf steps.
-template <bool kAny, bool kCount, bool kCurves>
-__device__ __forceinline__ void node_step(Traversal& T, const DevScene& S, uint2* stack,
-                                          uint32_t* err, Counters* cnt) {
-    if (kCurves && T.stage) curve_interior<kCount>(T, S, stack, err, cnt);
-    else trav_interior<kAny, kCount>(T, S, stack, err, cnt);
-}
+// Stage dispatch of the leaf step.
 template <bool kAny, bool kCount, bool kCurves, bool kMotion = false>
-__device__ __forceinline__ bool leaf_step(Traversal& T, const DevScene& S, uint32_t leaf, Counters* cnt) {
-    if (kCurves && T.stage) return curve_leaf_test<kAny, kCount>(T, S, leaf, cnt);
-    return leaf_test<kAny, kCount, kMotion>(T, S, leaf, cnt);
+__device__ __forceinline__ bool leaf_step(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack, Counters* cnt) {
+    if (kCurves && T.curve) return curve_leaf_test<kAny, kCount>(T, S, leaf, stack, cnt);
+    return leaf_test<kAny, kCount, kMotion>(T, S, leaf, stack, cnt);
 }
 
 // A lane whose triangle traversal ended moves on to the curve BVH (unless an
 // any-hit query already found a blocker). Returns true when the ray is done.
 template <bool kAny, bool kCurves>
-__device__ __forceinline__ bool stage_done(Traversal& T, float3 d, uint32_t segRoot) {
-    if (kCurves && T.stage == 0 && !(kAny && T.tri >= 0)) curve_begin(T, d, segRoot);
-    return T.exhausted;
+__device__ __forceinline__ bool stage_done(Traversal& T, uint2* stack) {
+    if (kCurves && !T.curve && !(kAny && T.prim != kNoPrim)) curve_begin(T, stack);
+    return T.cur == kEmptyChild;
 }
 
 // Done(i, T) consumes a finished traversal; Done(i, T, next) -> bool may
@@ -717,19 +770,12 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, uint32_t 
                                                     Counters* cnt, Load load, Done done) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t ltmask = (1u << lane) - 1u;
-    uint2 stack[kMaxStack4];
+    uint2 local[kFrame + kMaxStack4 + 1];
+    uint2* const stack = local + kFrame;
     Traversal T;
+    T.cur = kEmptyChild;  // of a lane without a ray, and of one whose traversal ended
     bool active = false, drained = false;
-    uint32_t idx = 0, parked = kEmptyChild;
-    // A queue shorter than the grid's lanes is dealt out evenly over all warps
-    // instead of 32 entries to the first ones: late bounces and small queries
-    // wait for their slowest warp, and a warp of few rays runs their diverging
-    // walks sooner than a full one. With at least 32 entries per warp nothing
-    // changes. 1280x720x8 hair frame: MIS stage (7 k rays per launch) 21.0 ->
-    // 12.2 ms; 960x540x1 pass of 938 spheres: 3.94 -> 3.29 ms; a query of 64
-    // rays 104 -> 78 us. Sharing what is left of a longer queue the same way
-    // (entries left / warps per refill) cost its extra atomics: Cornell
-    // 256x256x16 1.55 ms against 1.52.
+    uint32_t parked = kEmptyChild;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t share = (n - 1u) / warps + 1u;  // n = 0: any, nothing is fetched
     while (true) {
@@ -745,13 +791,12 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, uint32_t 
                 base = __shfl_sync(0xFFFFFFFFu, base, leader);
                 if (base >= n) drained = true;
                 if (!active) {
-                    const uint32_t rank = __popc(need & ltmask);
-                    idx = base + rank;
+                    const uint32_t rank = __popc(need & ltmask), idx = base + rank;
                     if (rank < take && idx < n) {
                         Ray ray;
                         uint32_t root, segRoot;
                         load(idx, ray, root, segRoot);
-                        trav_init(T, ray, root);
+                        trav_init<kCurves, kMotion>(T, ray, root, segRoot, idx, stack);
                         active = true;
                     }
                 }
@@ -760,51 +805,42 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, uint32_t 
         if (!__any_sync(0xFFFFFFFFu, active)) break;
         // 2. interior phase (speculative)
         while (true) {
-            if (kPark && active && !T.exhausted && (T.cur & 0x80000000u) && parked == kEmptyChild) {
+            if (kPark && int(T.cur) < 0 && T.cur != kEmptyChild && parked == kEmptyChild) {
                 parked = T.cur;
-                if (!trav_pop<kAny>(T, stack)) T.exhausted = true;
+                trav_pop<kAny>(T, stack);
             }
-            const bool want = active && !T.exhausted && !(T.cur & 0x80000000u);
-            const bool ready = !active || T.exhausted || (kPark ? parked != kEmptyChild : bool(T.cur & 0x80000000u));
+            const bool want = int(T.cur) >= 0;
             const uint32_t wantMask = __ballot_sync(0xFFFFFFFFu, want);
-            if (!wantMask || __all_sync(0xFFFFFFFFu, ready)) break;
+            if (!wantMask) break;
+            const bool leaf = kPark ? parked != kEmptyChild : !want && T.cur != kEmptyChild;
+            if (kPark && __all_sync(0xFFFFFFFFu, T.cur == kEmptyChild || leaf)) break;
             // Once at most kPhaseLanes lanes still descend and another lane
             // holds a leaf (any hit: a parked one), the phase ends and the
             // leaves are tested (the descending lanes resume in the next
             // interior phase), so few lanes do not hold the warp in the node
             // loop. A lane with a leaf must exist, so every pass makes progress.
-            constexpr uint32_t kPhaseLanes = kMotion ? 0u : (kPark ? kLeafPhaseLanesAny : kLeafPhaseLanes);
-            if (kPhaseLanes > 0 && __popc(wantMask) <= kPhaseLanes &&
-                __any_sync(0xFFFFFFFFu, active && !T.exhausted &&
-                                            (kPark ? parked != kEmptyChild : bool(T.cur & 0x80000000u))))
-                break;
+            constexpr int kPhaseLanes = kMotion ? 0 : (kPark ? kLeafPhaseLanesAny : kLeafPhaseLanes);
+            if (kPhaseLanes > 0 && __popc(wantMask) <= kPhaseLanes && __any_sync(0xFFFFFFFFu, leaf)) break;
             if (want) node_step<kAny, kCount, kCurves>(T, S, stack, err, cnt);
         }
         // 3. leaf phase: one leaf per lane
-        if (active) {
-            if (parked != kEmptyChild) {
-                if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, parked, cnt)) T.exhausted = true;
-                parked = kEmptyChild;
-            } else if (!T.exhausted && (T.cur & 0x80000000u)) {
-                if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, cnt)) T.exhausted = true;
-                else if (!trav_pop<kAny>(T, stack)) T.exhausted = true;
-            }
+        if (parked != kEmptyChild) {
+            if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, parked, stack, cnt)) T.cur = kEmptyChild;
+            parked = kEmptyChild;
+        } else if (int(T.cur) < 0 && T.cur != kEmptyChild) {
+            if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, stack, cnt)) T.cur = kEmptyChild;
+            else trav_pop<kAny>(T, stack);
         }
-        if (active && T.exhausted && parked == kEmptyChild) {
-            bool finished = true;
-            if (kCurves && T.stage == 0) {  // the curve BVH follows (the entry is read again for d)
-                Ray ray;
-                uint32_t root, segRoot;
-                load(idx, ray, root, segRoot);
-                finished = stage_done<kAny, kCurves>(T, ray.d, segRoot);
-            }
-            if (finished) {
+        if (active && T.cur == kEmptyChild && parked == kEmptyChild) {
+            if (stage_done<kAny, kCurves>(T, stack)) {  // else the curve BVH follows
+                trav_finish<kCurves>(T, stack);
+                const uint32_t idx = stack[-3].y;
                 Ray next;
                 if (trace_again(done, idx, T, next)) {
                     Ray ray;
                     uint32_t root, segRoot;
                     load(idx, ray, root, segRoot);
-                    trav_init(T, next, root);
+                    trav_init<kCurves, kMotion>(T, next, root, segRoot, idx, stack);
                 } else {
                     active = false;
                 }

@@ -51,3 +51,33 @@ def test_queue_lengths(gpu, restate_built, scene):
             check(r, po, rays[:n])
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("traversal", [api.ANA_TRAVERSAL_PER_RAY, api.ANA_TRAVERSAL_PERSISTENT],
+                         ids=["per_ray", "persistent"])
+def test_curve_rays_with_flat_components(gpu, restate_built, traversal):
+    """Rays through strands with one or two direction components of 0, -0 or
+    below 1e-9, which the curve boxes do not divide by, mixed with ordinary
+    rays of either sign in one warp."""
+    sc, _ = SCENES["hair"]
+    sc = sc()
+    rays = random_rays(4096, 1.6, 22)
+    rng = np.random.default_rng(23)
+    small = np.array([0.0, -0.0, 9e-10, -9e-10, 1e-9, -1e-9, 1e-12], np.float32)
+    for k in range(3):
+        rows = rng.random(len(rays)) < 0.35
+        rays[rows, 4 + k] = rng.choice(small, rows.sum())
+    keep = np.abs(rays[:, 4:7]).max(1) > 1e-3
+    rays = rays[keep]
+    rays[:, 4:7] /= np.linalg.norm(rays[:, 4:7].astype(np.float64), axis=1, keepdims=True)
+    # aim half of them at strand control points
+    cps = np.asarray(sc.control_points, np.float32).reshape(-1, 3)
+    half = len(rays) // 2
+    rays[:half, :3] = cps[rng.integers(0, len(cps), half)] - 0.5 * rays[:half, 4:7]
+    po = restate_built.PoScene(sc, 32)
+    r = api.Renderer(traversal=traversal)
+    try:
+        r.upload(sc)
+        check(r, po, rays)
+    finally:
+        r.close()
