@@ -152,11 +152,10 @@ __global__ void __launch_bounds__(256) k_generate(const __grid_constant__ Params
         const DevCamera& cam = R.cam;
         uint32_t px, py, sidx;
         path_coords(R, gid, px, py, sidx);
-        SampleStream ss{R.seed, px, py, sidx, 0};
-        float jx = ss.next(), jy = ss.next();
-        float lx = ss.next(), ly = ss.next();
-        float tu = ss.next();
-        (void)tu;  // shutter time: static scenes only
+        // dims 2 and 3 are read by a thin lens alone, dim 4 (the shutter time)
+        // by path_time
+        const float jx = radical_inverse2(sidx ^ halton_scramble(halton_pixel(R.seed, px, py), 0));
+        const float jy = halton_sample(R.seed, px, py, sidx, 1);
         float s = xdiv(xadd(__uint2float_rn(px), jx), __uint2float_rn(cam.width));
         float t = xdiv(xadd(__uint2float_rn(cam.height - 1u - py), jy), __uint2float_rn(cam.height));
         float3 target = xadd3(xadd3(cam.lower_left, xmul3(cam.horizontal, s)), xmul3(cam.vertical, t));
@@ -165,6 +164,7 @@ __global__ void __launch_bounds__(256) k_generate(const __grid_constant__ Params
             d = xnormalize(xsub3(target, o));
         } else {
             // thin lens, concentric disk mapping (IIntegrator.h:114-142)
+            const float lx = halton_sample(R.seed, px, py, sidx, 2), ly = halton_sample(R.seed, px, py, sidx, 3);
             float ax = 2.f * lx - 1.f, ay = 2.f * ly - 1.f, dx, dy;
             if (ax == 0.f && ay == 0.f) {
                 dx = dy = 0.f;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) k_generate(const __grid_constant__ Params
             o = lens;
             d = normalize(fp - lens);
         }
-        uint32_t meta = (ss.dim << 16);  // bounce 0, not specular
+        const uint32_t meta = 5u << 16;  // next dimension 5, bounce 0, not specular
         p.q.ext_o[0][i] = pack_u(o, gid);
         p.q.ext_d[0][i] = pack_u(d, meta);
         p.q.ext_b[0][i] = make_float4(1.f, 1.f, 1.f, __uint_as_float(sc));
@@ -540,12 +540,11 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
                         constexpr bool kShareSampler = (kFeat & kFeatStandard) != 0 || kFiber;
                         constexpr int kSampleUnroll = kShareSampler ? 1 : 2;
                         if (!m.is_delta && nL > 0) {
-                            float ul = ss.next();
-                            uint32_t lidx = min(uint32_t(ul * float(nL)), nL - 1u);
+                            const float3 lu = ss.next3();
+                            uint32_t lidx = min(uint32_t(lu.x * float(nL)), nL - 1u);
                             L = S.lights[R.light_base + lidx];
                             // light sampling
-                            float lu0 = ss.next(), lu1 = ss.next();
-                            LightSample ls = light_sample<kFeat>(S, L, si.p, lu0, lu1);
+                            LightSample ls = light_sample<kFeat>(S, L, si.p, lu.y, lu.z);
                             if (ls.pdf > 0.f && !is_black(ls.Li)) {
                                 BsdfEval be = mat_eval<kFiber, kExtra, kFeat>(m, c, wo, ls.wi);
                                 if (!is_black(be.f)) {
@@ -600,9 +599,8 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
 #pragma unroll (kSampleUnroll)
                         for (int k = kShareSampler ? (misPending ? 0 : 1) : 0; k < 2; ++k) {
                             if (!kShareSampler && k == 0 && !misPending) continue;
-                            const float uc = ss.next();
-                            const float u0 = ss.next(), u1 = ss.next();
-                            BsdfSample bs = mat_sample<kFiber, kExtra, kFeat>(m, c, wo, u0, u1, uc);
+                            const float3 us = ss.next3();
+                            BsdfSample bs = mat_sample<kFiber, kExtra, kFeat>(m, c, wo, us.y, us.z, us.x);
                             if (!bs.valid()) continue;
                             if (k == 0) {
                                 float lp = light_pdf<kFeat>(S, L, si.p, bs.wi);
