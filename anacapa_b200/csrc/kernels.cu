@@ -249,7 +249,7 @@ __device__ __forceinline__ void warp_add_work(unsigned long long* work, const Co
 //   kPersist: persistent warps with per-lane refill (persistent_traverse);
 //   otherwise one thread per ray over a grid-stride loop.
 // Both use the same interior/leaf steps, so results are identical.
-template <bool kAny, bool kCount, bool kPersist, bool kCurves, bool kMotion = false, bool kPark = kAny,
+template <bool kAny, bool kCount, bool kPersist, bool kCurves, bool kMotion = false, bool kPark = kAny && !kCurves,
           class Load, class Done>
 __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uint32_t* fetch, uint32_t* err,
                                               Counters* cnt, Load load, Done done) {
@@ -258,6 +258,7 @@ __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uin
     } else {
         uint2 local[kFrame + kMaxStack4 + 1];
         uint2* const stack = local + kFrame;
+        SubSeg ribbon[kCurves ? kRibbonStack : 1];
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             Ray ray;
             uint32_t root, segRoot;
@@ -268,8 +269,7 @@ __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uin
                 do {
                     while (T.cur != kEmptyChild) {
                         if (int(T.cur) >= 0) node_step<kAny, kCount, kCurves>(T, S, stack, err, cnt);
-                        else if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, stack, cnt)) T.cur = kEmptyChild;
-                        else trav_pop<kAny>(T, stack);
+                        else leaf_step<kAny, kCount, kCurves, kMotion>(T, S, stack, ribbon, cnt);
                     }
                 } while (!stage_done<kAny, kCurves>(T, stack));
                 trav_finish<kCurves>(T, stack);
@@ -285,7 +285,7 @@ __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uin
 // spills (1920x1080x64 throughput frame: 290.2 ms; 293.8 at 56 registers and
 // 36 warps per SM, 292.2 at 40 and 48 warps); the motion variants (object-ray
 // state) keep 4 and 64 registers; with the curve stage they take 3 and 80 (the
-// ribbon test's state; 1280x720x8 hair frame 260.0 ms against 285.1 at 4
+// ribbon walk's state; 1280x720x8 hair frame 172.2 ms against 178.9 at 4
 // blocks and 64 registers).
 #define ANA_TRAVERSAL_BOUNDS \
     __launch_bounds__(kPersistBlock, kPersist ? (kCurves ? 3 : (kMotion ? 4 : kPersistMinBlocks)) : 1)
@@ -745,12 +745,11 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
 // opaque scenes — any blocker in [1e-4, tmax] makes the transmittance black.
 // Triangle-only batches test each leaf as they reach it (1920x1080x64
 // throughput frame: shadow stage 53.1 ms parking leaves, 46.3 ms without; the
-// motion frame 45.8 -> 42.1 ms); with curves the lanes park leaves (the hair
-// frame's shadow stage 373.0 against 374.3 ms).
+// motion frame 45.8 -> 42.1 ms), as do those with curves.
 template <bool kCurves, bool kPersist, bool kAdj, bool kMotion = false>
 __global__ void ANA_TRAVERSAL_BOUNDS k_shadow(const __grid_constant__ Params p) {
     uint32_t* cb = p.counters + p.bounce * kCountersPerBounce;
-    run_traversal<true, false, kPersist, kCurves, kMotion, kCurves>(
+    run_traversal<true, false, kPersist, kCurves, kMotion, false>(
         p.S, cb[1], cb + 4, p.err, nullptr,
         [&](uint32_t i, Ray& r, uint32_t& root, uint32_t& segRoot) {
             float4 o = p.q.sh_o[i], d = p.q.sh_d[i];

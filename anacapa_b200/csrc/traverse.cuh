@@ -129,9 +129,10 @@ struct Counters {
 //      shortens the ray and culls later nodes (measured on the throughput
 //      frame: speculation cost closest hit 3 %, saved any hit 8-12 % with
 //      one-lane refills; with grouped refills it costs the triangle shadow
-//      and MIS kernels too, and only the curve shadow kernels and the
-//      occlusion queries of ana_trace_batch park);
-//   3. leaf phase: the parked leaf's (else the current leaf's) triangles.
+//      and MIS kernels too, and only the occlusion queries of ana_trace_batch
+//      on triangles park);
+//   3. leaf phase: the parked leaf's (else the current leaf's) triangles; curve
+//      leaves begin and walk their segments in steps of their own.
 // A lane whose stack is used up (or, for occlusion, that found a blocker)
 // reports its ray and picks up a new one at the next refill, so finished rays
 // do not idle the warp until its slowest ray completes. Box and triangle
@@ -144,13 +145,26 @@ struct Counters {
 // refilling one lane at a time, 146.5 ms, 137.0 at 4, 132.8 at 8, 128.1 at 16,
 // 129.8 at 24 and 191.2 at 32. Any-hit kernels that test leaves as reached use
 // the closest-hit count (shadow + MIS 107.0 ms at 8, 111.4 at 4, 108.1 at 12,
-// 111.9 at 16); the parked count serves the kernels that still park (curve
-// shadow rays, occlusion queries of ana_trace_batch). Kernels with
+// 111.9 at 16); the parked count serves the kernels that still park
+// (occlusion queries of ana_trace_batch on triangles). Kernels with
 // motion-blurred meshes, whose leaf tests invert interpolated matrices, keep
 // the phase until no lane descends (1280x720x16 motion frame: 25.9 ms against
 // 28.6 ms at 8 / 16 lanes). Hits and occlusion answers are unchanged.
 constexpr uint32_t kLeafPhaseLanes = 8;      // closest hit, any hit without parking
 constexpr uint32_t kLeafPhaseLanesAny = 16;  // any hit (parked leaves)
+
+// Curve leaves: lanes with a segment to begin do so together, lanes inside a
+// ribbon walk step together once kWalkLanes of them wait (or nothing else is
+// left to do), and the phase ends when at most kBeginLanes segments wait to
+// begin. A lane that walked its segment alone held the warp for up to 64 leaves
+// of the walk, with 4 of 32 lanes active. 1280x720x8 hair frame, closest-hit
+// stage: 145.9 ms a whole segment per lane at a time, 130.6 one node per lane
+// and phase; with most segments rejected before their walk (ribbon_far) 102.2,
+// and 98.7 with begin and walk steps apart (kWalkLanes 4: 100.5, 6: 98.7, 8:
+// 98.7, 12: 102.2; kBeginLanes 4: 101.4 and 12: 99.3; interior phases ending
+// at 6 or 10 lanes instead of 8: 100.5, 98.0).
+constexpr int kWalkLanes = 6;
+constexpr int kBeginLanes = 8;
 
 // Refill thresholds: idle lanes take new rays only once at least this many
 // lanes of the warp are idle (or the queue is drained and every lane is).
@@ -176,9 +190,12 @@ struct Traversal {
     uint32_t prim;   // closest hit so far: leaf-order triangle, 0x80000000 | segment, or kNoPrim
     uint32_t cur;
     int sp;
+    int rs;          // curve stage: nodes on the stack of the current segment's ribbon walk
     // curve stage (scenes with curves): the triangle BVH is traversed first,
     // then the curve BVH from the triangle hit distance (CurveBrute::trace)
     bool curve;      // the curve BVH is being traversed
+    bool unit;       // the direction has unit length (ribbon_far's margin)
+    float margin;    // ribbon_far's, of the current segment
     bool flat;       // a direction component is below CurveBrute::aabbHit's 1e-9
     // filled from the frame when the ray is reported
     float u, v, tseg;
@@ -222,6 +239,7 @@ __device__ __forceinline__ void trav_init(Traversal& T, const Ray& ray, uint32_t
     T.cur = root;
     T.sp = 1;
     stack[0] = make_uint2(kEmptyChild, __float_as_uint(-INFINITY));
+    T.rs = 0;
     T.curve = false;
     T.flat = false;
     const float3 d = tri_dir(T.r);
@@ -585,26 +603,25 @@ struct SubSeg {
     uint32_t dp;            // depth (bits 0-2, 6 = root) | path from the root (bits 3-8, 1 = right)
 };
 
-// The half-widths and strand-parameter interval of the node (depth, path)
-// below a segment's (hw0r, hw3r, toffr, tscr): the splits' own updates
-// (CurveBrute.cpp:152-176) replayed from the root.
-__device__ __forceinline__ void ribbon_params(uint32_t dp, float hw0r, float hw3r, float toffr, float tscr,
-                                              float& hw0, float& hw3, float& toff, float& tscale) {
-    const int levels = 6 - int(dp & 7u);
-    const uint32_t path = dp >> 3;
+// The half-widths, and the strand-parameter interval, of the node (depth,
+// path) below a segment's: the splits' own updates (CurveBrute.cpp:152-176)
+// replayed from the root.
+__device__ __forceinline__ void ribbon_widths(uint32_t dp, float hw0r, float hw3r, float& hw0, float& hw3) {
     hw0 = hw0r;
     hw3 = hw3r;
+    for (int k = 5 - int(dp & 7u); k >= 0; --k) {
+        const float hm = xmul(xadd(hw0, hw3), 0.5f);
+        if ((dp >> (3 + k)) & 1u) hw0 = hm;
+        else hw3 = hm;
+    }
+}
+__device__ __forceinline__ void ribbon_interval(uint32_t dp, float toffr, float tscr, float& toff, float& tscale) {
     toff = toffr;
     tscale = tscr;
-    for (int k = levels - 1; k >= 0; --k) {
-        const float hm = xmul(xadd(hw0, hw3), 0.5f), tsh = xmul(tscale, 0.5f);
-        if ((path >> k) & 1u) {
-            hw0 = hm;
-            toff = xadd(toff, tsh);
-        } else {
-            hw3 = hm;
-        }
-        tscale = tsh;
+    for (int k = 5 - int(dp & 7u); k >= 0; --k) {
+        const float half = xmul(tscale, 0.5f);
+        if ((dp >> (3 + k)) & 1u) toff = xadd(toff, half);
+        tscale = half;
     }
 }
 
@@ -624,61 +641,123 @@ __device__ __forceinline__ void ribbon_params(uint32_t dp, float hw0r, float hw3
 // 398.6 -> 379.3 ms). (A walk that kept no points at all, rebuilding each
 // right half from the segment's four points along its path, measured slower:
 // extend 1024 against 842 ms at leaves of four.)
-__device__ __forceinline__ bool ribbon_hit(const RayFrame& fr, float tmin, float3 P0, float3 P1, float3 P2,
-                                           float3 P3, float hw0r, float hw3r, float toffr, float tscaler,
-                                           float& bestT, float& tSeg, float3& tang) {
-    SubSeg st[8];
-    int sp = 0;
-    {
-        const float3 c0 = project(fr, P0), c1 = project(fr, P1), c2 = project(fr, P2), c3 = project(fr, P3);
-        float zlo;
-        if (!ribbon_bounds(c0, c1, c2, c3, hw0r, hw3r, tmin, bestT, zlo)) return false;
-        st[sp++] = SubSeg{P0, P1, P2, P3, zlo, 6u};
+constexpr int kRibbonStack = 8;
+
+// Whether no leaf of the walk below a node can be hit: its projected control
+// points all lie on one side of the ray axis, further from it than r along the
+// normal of the chord, so does their hull, and so every chord of a leaf. r is
+// the larger half-width plus a margin for the rounding of the walk's own
+// arithmetic: its midpoints round 18 times on coordinates up to |P|, a
+// projection 6 times on |P| + |o|, the leaf's distance a few times more, in all
+// below 4e-6 (|P| + |o|) for a direction of unit length; the margin is 1e-5 of
+// it. A rejected segment therefore never had a hit to report, and results are
+// unchanged. The walk's own bounds (a box in ray space, axis-aligned) pass two
+// thirds of the segments that a ray meets, though a strand's segment is thin
+// and lies at any angle: with this test before them a ray of the hair frame
+// walks 13 nodes instead of 82.
+__device__ __forceinline__ bool ribbon_far(float3 c0, float3 c1, float3 c2, float3 c3, float r) {
+    const float ux = c3.x - c0.x, uy = c3.y - c0.y;
+    const float s0 = c0.y * ux - c0.x * uy, s1 = c1.y * ux - c1.x * uy, s2 = c2.y * ux - c2.x * uy,
+                s3 = c3.y * ux - c3.x * uy;
+    const float d = fmaxf(min4(s0, s1, s2, s3), -max4(s0, s1, s2, s3));
+    const float rl = r * r * (ux * ux + uy * uy);
+    return d > 0.f && rl > 1e-30f && d * d > rl;
+}
+__device__ __forceinline__ float norm1(float3 p) { return fabsf(p.x) + fabsf(p.y) + fabsf(p.z); }
+
+// The ray frame (ray origin, x and y axes, direction) from the lane's frame.
+__device__ __forceinline__ RayFrame ray_frame(const Traversal& T, const uint2* stack) {
+    const uint2 a = stack[-4], b = stack[-5], c = stack[-6];
+    return RayFrame{T.r.o, f3(lo(a), hi(a), lo(b)), f3(hi(b), lo(c), hi(c)), frame_dir(stack)};
+}
+
+// Begins the current leaf's first segment: a survivor of the tests of the whole
+// segment is the walk's first node.
+__device__ __forceinline__ void ribbon_start(Traversal& T, const DevScene& S, const uint2* stack, SubSeg* st) {
+    const RayFrame fr = ray_frame(T, stack);
+    const float4* sp4 = S.segs + 5 * size_t(T.cur & 0x01FFFFFFu);
+    const float4 a = ldg4(sp4), b = ldg4(sp4 + 1), e = ldg4(sp4 + 2), g = ldg4(sp4 + 3);
+    const float3 P0 = f3(a), P1 = f3(b), P2 = f3(e), P3 = f3(g);
+    T.margin = T.unit ? 1e-5f * (max4(norm1(P0), norm1(P1), norm1(P2), norm1(P3)) + norm1(fr.o)) : INFINITY;
+    T.rs = 0;
+    // fused arithmetic: the margin covers it, and most segments end here
+    // without the walk's separately rounded projections (1280x720x8 hair frame:
+    // closest-hit stage 130.6 -> 102.2 ms, 107.2 with the test after those)
+    const float3 q0 = P0 - fr.o, q1 = P1 - fr.o, q2 = P2 - fr.o, q3 = P3 - fr.o;
+    if (ribbon_far(f3(dot(q0, fr.x), dot(q0, fr.y), 0.f), f3(dot(q1, fr.x), dot(q1, fr.y), 0.f),
+                   f3(dot(q2, fr.x), dot(q2, fr.y), 0.f), f3(dot(q3, fr.x), dot(q3, fr.y), 0.f),
+                   fmaxf(fabsf(a.w), fabsf(b.w)) * 1.00001f + T.margin))
+        return;
+    const float3 c0 = project(fr, P0), c1 = project(fr, P1), c2 = project(fr, P2), c3 = project(fr, P3);
+    float zlo;
+    if (ribbon_bounds(c0, c1, c2, c3, a.w, b.w, T.r.tmin, T.closest, zlo))
+        st[T.rs++] = SubSeg{P0, P1, P2, P3, zlo, 6u};
+}
+
+// One node of the walk of the current leaf's first segment. True when it is a
+// closer hit (recorded).
+template <bool kAny>
+__device__ __forceinline__ bool ribbon_step(Traversal& T, const DevScene& S, uint2* stack, SubSeg* st) {
+    const SubSeg s = st[--T.rs];
+    if (s.zlo > T.closest) return false;
+    const RayFrame fr = ray_frame(T, stack);
+    const uint32_t seg = T.cur & 0x01FFFFFFu;
+    const float* sw = reinterpret_cast<const float*>(S.segs + 5 * size_t(seg)) + 3;
+    float hw0, hw3;
+    ribbon_widths(s.dp, __ldg(sw), __ldg(sw + 4), hw0, hw3);
+    const float3 c0 = project(fr, s.P0), c3 = project(fr, s.P3);
+    if ((s.dp & 7u) == 0u) {
+        const float ax = c0.x, ay = c0.y, bx = c3.x, by = c3.y;
+        const float dx = xsub(bx, ax), dy = xsub(by, ay);
+        const float lenSq = xadd(xmul(dx, dx), xmul(dy, dy));
+        float tLine;
+        if (lenSq < 1e-12f) tLine = 0.f;
+        else
+            tLine = fmaxf(0.f, fminf(1.f, xdiv(xsub(xmul(-ax, dx), xmul(ay, dy)), lenSq)));
+        const float px = xadd(ax, xmul(dx, tLine)), py = xadd(ay, xmul(dy, tLine));
+        const float dist2 = xadd(xmul(px, px), xmul(py, py));
+        const float halfW = xadd(xmul(hw0, xsub(1.f, tLine)), xmul(hw3, tLine));
+        if (dist2 > xmul(halfW, halfW)) return false;
+        const float tRay = xadd(c0.z, xmul(xsub(c3.z, c0.z), tLine));
+        if (tRay < T.r.tmin || tRay >= T.closest) return false;
+        T.closest = tRay;
+        T.prim = 0x80000000u | seg;
+        if (kAny) return true;
+        float3 tg = bezier_tangent(s.P0, s.P1, s.P2, s.P3, tLine);
+        if (xdot(tg, tg) < 1e-12f) tg = xsub3(s.P3, s.P0);
+        const float len = __fsqrt_rn(xdot(tg, tg));
+        tg = len > 1e-8f ? xmul3(tg, xdiv(1.f, len)) : f3(0.f, 0.f, 1.f);
+        float toff, tscale;
+        ribbon_interval(s.dp, __ldg(sw + 8), __ldg(sw + 12), toff, tscale);
+        stack[-7] = pair(tg.x, tg.y);
+        stack[-8] = pair(tg.z, xadd(toff, xmul(tLine, tscale)));
+        return true;
     }
-    bool hit = false;
-    while (sp > 0) {
-        const SubSeg s = st[--sp];
-        if (s.zlo > bestT) continue;
-        float hw0, hw3, toff, tscale;
-        ribbon_params(s.dp, hw0r, hw3r, toffr, tscaler, hw0, hw3, toff, tscale);
-        const float3 c0 = project(fr, s.P0), c3 = project(fr, s.P3);
-        if ((s.dp & 7u) == 0u) {
-            const float ax = c0.x, ay = c0.y, bx = c3.x, by = c3.y;
-            const float dx = xsub(bx, ax), dy = xsub(by, ay);
-            const float lenSq = xadd(xmul(dx, dx), xmul(dy, dy));
-            float tLine;
-            if (lenSq < 1e-12f) tLine = 0.f;
-            else
-                tLine = fmaxf(0.f, fminf(1.f, xdiv(xsub(xmul(-ax, dx), xmul(ay, dy)), lenSq)));
-            const float px = xadd(ax, xmul(dx, tLine)), py = xadd(ay, xmul(dy, tLine));
-            const float dist2 = xadd(xmul(px, px), xmul(py, py));
-            const float halfW = xadd(xmul(hw0, xsub(1.f, tLine)), xmul(hw3, tLine));
-            if (dist2 > xmul(halfW, halfW)) continue;
-            const float tRay = xadd(c0.z, xmul(xsub(c3.z, c0.z), tLine));
-            if (tRay < tmin || tRay >= bestT) continue;
-            float3 tg = bezier_tangent(s.P0, s.P1, s.P2, s.P3, tLine);
-            if (xdot(tg, tg) < 1e-12f) tg = xsub3(s.P3, s.P0);
-            const float len = __fsqrt_rn(xdot(tg, tg));
-            tg = len > 1e-8f ? xmul3(tg, xdiv(1.f, len)) : f3(0.f, 0.f, 1.f);
-            bestT = tRay;
-            tSeg = xadd(toff, xmul(tLine, tscale));
-            tang = tg;
-            hit = true;
-            continue;
-        }
-        const float3 Q01 = xmid(s.P0, s.P1), Q12 = xmid(s.P1, s.P2), Q23 = xmid(s.P2, s.P3);
-        const float3 R01 = xmid(Q01, Q12), R12 = xmid(Q12, Q23), M = xmid(R01, R12);
-        const float3 cq01 = project(fr, Q01), cr01 = project(fr, R01), cm = project(fr, M),
-                     cr12 = project(fr, R12), cq23 = project(fr, Q23);
-        const float hwMid = xmul(xadd(hw0, hw3), 0.5f);
-        float zl, zr;
-        const bool okL = ribbon_bounds(c0, cq01, cr01, cm, hw0, hwMid, tmin, bestT, zl);
-        const bool okR = ribbon_bounds(cm, cr12, cq23, c3, hwMid, hw3, tmin, bestT, zr);
-        const uint32_t cd = (s.dp & 7u) - 1u, cp = (s.dp >> 3) << 1;
-        if (okR) st[sp++] = SubSeg{M, R12, Q23, s.P3, zr, cd | ((cp | 1u) << 3)};
-        if (okL) st[sp++] = SubSeg{s.P0, Q01, R01, M, zl, cd | (cp << 3)};
+    const float3 Q01 = xmid(s.P0, s.P1), Q12 = xmid(s.P1, s.P2), Q23 = xmid(s.P2, s.P3);
+    const float3 R01 = xmid(Q01, Q12), R12 = xmid(Q12, Q23), M = xmid(R01, R12);
+    const float3 cq01 = project(fr, Q01), cr01 = project(fr, R01), cm = project(fr, M), cr12 = project(fr, R12),
+                 cq23 = project(fr, Q23);
+    const float hwMid = xmul(xadd(hw0, hw3), 0.5f);
+    float zl, zr;
+    bool okL = ribbon_bounds(c0, cq01, cr01, cm, hw0, hwMid, T.r.tmin, T.closest, zl);
+    bool okR = ribbon_bounds(cm, cr12, cq23, c3, hwMid, hw3, T.r.tmin, T.closest, zr);
+    const uint32_t cd = (s.dp & 7u) - 1u, cp = (s.dp >> 3) << 1;
+    if (!kAny) {  // closest hit 109.1 -> 107.1 ms; any hit, which ends at its first leaf, 65.6 -> 69.6
+        const float rf = fmaxf(fabsf(hw0), fabsf(hw3)) * 1.00001f + T.margin;
+        okL = okL && !ribbon_far(c0, cq01, cr01, cm, rf);
+        okR = okR && !ribbon_far(cm, cr12, cq23, c3, rf);
     }
-    return hit;
+    if (okR) st[T.rs++] = SubSeg{M, R12, Q23, s.P3, zr, cd | ((cp | 1u) << 3)};
+    if (okL) st[T.rs++] = SubSeg{s.P0, Q01, R01, M, zl, cd | (cp << 3)};
+    return false;
+}
+
+// The segment's walk is over: on to the leaf's next segment, else the next
+// stack entry.
+template <bool kAny>
+__device__ __forceinline__ void ribbon_next(Traversal& T, const uint2* stack) {
+    if (((T.cur >> 25) & 63u) != 0u) T.cur = T.cur - (1u << 25) + 1u;
+    else trav_pop<kAny>(T, stack);
 }
 
 // ---------------------------------------------------------------------------
@@ -696,6 +775,7 @@ __device__ __forceinline__ void curve_begin(Traversal& T, uint2* stack) {
     onb_exact(d, fx, fy);
     T.curve = true;
     T.flat = fabsf(d.x) < 1e-9f || fabsf(d.y) < 1e-9f || fabsf(d.z) < 1e-9f;
+    T.unit = fabsf(dot(d, d) - 1.f) < 1e-3f;
     T.r.inv = f3(xdiv(1.f, d.x), xdiv(1.f, d.y), xdiv(1.f, d.z));
     T.cur = segRoot;
     T.sp = 1;  // stack[0] still ends the stack
@@ -706,35 +786,25 @@ __device__ __forceinline__ void curve_begin(Traversal& T, uint2* stack) {
     stack[-6] = pair(fy.y, fy.z);
 }
 
-// Ribbon tests of one curve leaf; true when an any-hit query found its blocker.
-template <bool kAny, bool kCount>
-__device__ __forceinline__ bool curve_leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack,
-                                                Counters* cnt) {
-    const uint2 p4 = stack[-4], p5 = stack[-5], p6 = stack[-6];
-    const RayFrame fr{T.r.o, f3(lo(p4), hi(p4), lo(p5)), f3(hi(p5), lo(p6), hi(p6)), frame_dir(stack)};
-    const uint32_t off = leaf & 0x01FFFFFFu, c = ((leaf >> 25) & 63u) + 1u;
-    for (uint32_t i = off; i < off + c; ++i) {
-        const float4* sp4 = S.segs + 5 * size_t(i);
-        const float4 a = ldg4(sp4), b = ldg4(sp4 + 1), e = ldg4(sp4 + 2), g = ldg4(sp4 + 3);
-        if (kCount) cnt->segs++;
-        float ts, bt = T.closest;
-        float3 tg;
-        if (ribbon_hit(fr, T.r.tmin, f3(a), f3(b), f3(e), f3(g), a.w, b.w, e.w, g.w, bt, ts, tg)) {
-            T.prim = 0x80000000u | i;
-            T.closest = bt;
-            if (kAny) return true;
-            stack[-7] = pair(tg.x, tg.y);
-            stack[-8] = pair(tg.z, ts);
-        }
-    }
-    return false;
-}
-
-// Stage dispatch of the leaf step.
+// A whole leaf at once, and the step after it (one-thread-per-ray schedule;
+// triangle leaves of the persistent one).
 template <bool kAny, bool kCount, bool kCurves, bool kMotion = false>
-__device__ __forceinline__ bool leaf_step(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack, Counters* cnt) {
-    if (kCurves && T.curve) return curve_leaf_test<kAny, kCount>(T, S, leaf, stack, cnt);
-    return leaf_test<kAny, kCount, kMotion>(T, S, leaf, stack, cnt);
+__device__ __forceinline__ void leaf_step(Traversal& T, const DevScene& S, uint2* stack, SubSeg* st, Counters* cnt) {
+    if (kCurves && T.curve) {
+        if (kCount) cnt->segs++;
+        ribbon_start(T, S, stack, st);
+        while (T.rs > 0) {
+            if (ribbon_step<kAny>(T, S, stack, st) && kAny) {
+                T.cur = kEmptyChild;
+                return;
+            }
+        }
+        ribbon_next<kAny>(T, stack);
+    } else if (leaf_test<kAny, kCount, kMotion>(T, S, T.cur, stack, cnt)) {
+        T.cur = kEmptyChild;
+    } else {
+        trav_pop<kAny>(T, stack);
+    }
 }
 
 // A lane whose triangle traversal ended moves on to the curve BVH (unless an
@@ -772,10 +842,22 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, uint32_t 
     const uint32_t ltmask = (1u << lane) - 1u;
     uint2 local[kFrame + kMaxStack4 + 1];
     uint2* const stack = local + kFrame;
+    SubSeg ribbon[kCurves ? kRibbonStack : 1];
     Traversal T;
+    T.rs = 0;
+    T.curve = false;
     T.cur = kEmptyChild;  // of a lane without a ray, and of one whose traversal ended
     bool active = false, drained = false;
     uint32_t parked = kEmptyChild;
+    // A queue shorter than the grid's lanes is dealt out evenly over all warps
+    // instead of 32 entries to the first ones: late bounces and small queries
+    // wait for their slowest warp, and a warp of few rays runs their diverging
+    // walks sooner than a full one. With at least 32 entries per warp nothing
+    // changes. 1280x720x8 hair frame: MIS stage (7 k rays per launch) 21.0 ->
+    // 12.2 ms; 960x540x1 pass of 938 spheres: 3.94 -> 3.29 ms; a query of 64
+    // rays 104 -> 78 us. Sharing what is left of a longer queue the same way
+    // (entries left / warps per refill) cost its extra atomics: Cornell
+    // 256x256x16 1.55 ms against 1.52.
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t share = (n - 1u) / warps + 1u;  // n = 0: any, nothing is fetched
     while (true) {
@@ -819,17 +901,42 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, uint32_t 
             // leaves are tested (the descending lanes resume in the next
             // interior phase), so few lanes do not hold the warp in the node
             // loop. A lane with a leaf must exist, so every pass makes progress.
-            constexpr int kPhaseLanes = kMotion ? 0 : (kPark ? kLeafPhaseLanesAny : kLeafPhaseLanes);
+            constexpr int kPhaseLanes = kMotion && !kCurves ? 0 : (kPark ? kLeafPhaseLanesAny : kLeafPhaseLanes);
             if (kPhaseLanes > 0 && __popc(wantMask) <= kPhaseLanes && __any_sync(0xFFFFFFFFu, leaf)) break;
             if (want) node_step<kAny, kCount, kCurves>(T, S, stack, err, cnt);
         }
-        // 3. leaf phase: one leaf per lane
-        if (parked != kEmptyChild) {
-            if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, parked, stack, cnt)) T.cur = kEmptyChild;
+        // 3. leaf phase: one triangle leaf per lane
+        if (kPark && parked != kEmptyChild) {
+            if (leaf_test<kAny, kCount, kMotion>(T, S, parked, stack, cnt)) T.cur = kEmptyChild;
             parked = kEmptyChild;
-        } else if (int(T.cur) < 0 && T.cur != kEmptyChild) {
-            if (leaf_step<kAny, kCount, kCurves, kMotion>(T, S, T.cur, stack, cnt)) T.cur = kEmptyChild;
-            else trav_pop<kAny>(T, stack);
+        } else if (int(T.cur) < 0 && T.cur != kEmptyChild && !(kCurves && T.curve)) {
+            leaf_step<kAny, kCount, false, kMotion>(T, S, stack, nullptr, cnt);
+        }
+        // curve leaves: every lane with a segment starts it or walks one node
+        if (kCurves) {
+            bool acted = false;  // every phase begins or walks at least once
+            while (true) {
+                const bool leaf = T.curve && int(T.cur) < 0 && T.cur != kEmptyChild;
+                const bool walk = T.rs > 0, begin = leaf && !walk;
+                const uint32_t beginMask = __ballot_sync(0xFFFFFFFFu, begin);
+                const int walks = __popc(__ballot_sync(0xFFFFFFFFu, walk));
+                if (acted && walks < kWalkLanes && __popc(beginMask) <= kBeginLanes) break;
+                if (walks >= kWalkLanes || !beginMask) {
+                    if (walk) {
+                        if (ribbon_step<kAny>(T, S, stack, ribbon) && kAny) {
+                            T.rs = 0;
+                            T.cur = kEmptyChild;
+                        } else if (T.rs == 0) {
+                            ribbon_next<kAny>(T, stack);
+                        }
+                    }
+                } else if (begin) {
+                    if (kCount) cnt->segs++;
+                    ribbon_start(T, S, stack, ribbon);
+                    if (T.rs == 0) ribbon_next<kAny>(T, stack);
+                }
+                acted = true;
+            }
         }
         if (active && T.cur == kEmptyChild && parked == kEmptyChild) {
             if (stage_done<kAny, kCurves>(T, stack)) {  // else the curve BVH follows

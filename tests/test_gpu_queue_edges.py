@@ -2,6 +2,9 @@
 schedule changes how it deals out entries (one per warp, a warp's 32 lanes,
 ragged lengths), against the CPU restatement in float: the same ids and
 distances, ties within 1e-6 relative t aside."""
+import dataclasses
+import hashlib
+
 import numpy as np
 import pytest
 
@@ -79,5 +82,47 @@ def test_curve_rays_with_flat_components(gpu, restate_built, traversal):
     try:
         r.upload(sc)
         check(r, po, rays)
+    finally:
+        r.close()
+
+
+@pytest.mark.parametrize("traversal", [api.ANA_TRAVERSAL_PER_RAY, api.ANA_TRAVERSAL_PERSISTENT],
+                         ids=["per_ray", "persistent"])
+@pytest.mark.parametrize("scale,shift,stretch", [(1.0, 0.0, 1.0), (1.0, 1000.0, 1.0), (1e-3, 0.0, 1.0),
+                                                 (500.0, 0.0, 1.0), (1.0, 0.0, 0.37), (1.0, 0.0, 25.0)],
+                         ids=["plain", "far_from_origin", "tiny", "large", "short_direction", "long_direction"])
+def test_rays_at_ribbon_edges(gpu, restate_built, scale, shift, stretch, traversal):
+    """Rays past strands at distances around the half-width, where a segment
+    may only be rejected unseen if no leaf of its walk is hit: strands far from
+    the origin, tiny and large, thin and wide, against the restatement. For
+    directions that are not of unit length a ribbon's distance and a box's are
+    in different units, and what is found depends on the order of the visits;
+    there the answers are those of the walk without any rejection, recorded."""
+    sc = S.hair(64, 36, 1, n_strands=600)
+    cps = np.asarray(sc.control_points, np.float32).reshape(-1, 3) * np.float32(scale) + np.float32(shift)
+    widths = np.asarray(sc.widths, np.float32) * np.float32(scale)
+    widths[::4] *= np.float32(20.0)
+    sc = dataclasses.replace(sc, control_points=cps, widths=widths, area_lights=[])
+    rng = np.random.default_rng(24)
+    n = 1 << 15
+    at = rng.integers(0, 600, n) * 13 + rng.integers(1, 12, n)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    p = cps.astype(np.float64)
+    side = np.cross(d, p[at + 1] - p[at - 1])
+    side /= np.maximum(np.linalg.norm(side, axis=1, keepdims=True), 1e-30)
+    off = 0.5 * widths.reshape(-1, 2)[at // 13].mean(1) * rng.choice([0.0, 0.3, 0.9, 0.999, 1.0, 1.001, 1.1, 1.5], n)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, :3] = p[at] + side * off[:, None] - d * (scale * rng.uniform(0.01, 2.0, (n, 1)))
+    rays[:, 4:7] = d * stretch
+    rays[:, 3], rays[:, 7] = 1e-4 * scale, 1e10
+    r = api.Renderer(traversal=traversal)
+    try:
+        r.upload(sc)
+        if stretch == 1.0:
+            check(r, restate_built.PoScene(sc, 32), rays)
+        else:
+            found = [hashlib.sha1(r.trace(rays, occlusion=o).tobytes()).hexdigest()[:10] for o in (False, True)]
+            assert found == {0.37: ["47406624bd", "de8dd33e3e"], 25.0: ["ac511829ec", "f4250bde8c"]}[stretch]
     finally:
         r.close()
