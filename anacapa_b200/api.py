@@ -420,8 +420,8 @@ class Renderer:
 
     def aovs(self, width, height):
         """ana_aov_read: resolved first-hit albedo and shading normal, (H, W, 3) each."""
-        al = np.zeros((height, width, 3), np.float32)
-        nr = np.zeros((height, width, 3), np.float32)
+        al = np.empty((height, width, 3), np.float32)
+        nr = np.empty((height, width, 3), np.float32)
         self._check(lib().ana_aov_read(self.h, al.ctypes.data, nr.ctypes.data, width * height))
         return al, nr
 
@@ -454,7 +454,7 @@ class Renderer:
 
     def film(self, width, height) -> np.ndarray:
         """(H, W, 5) float32: pre-weighted r, g, b, weight, sum of lum^2."""
-        out = np.zeros((height, width, 5), np.float32)
+        out = np.empty((height, width, 5), np.float32)
         self._check(lib().ana_film_read(self.h, out.ctypes.data, width * height))
         return out
 
@@ -499,7 +499,7 @@ class Renderer:
                     if v is not None}
             st = self._diff_struct(keep)
         r = AnaRenderDesc(width, height, sample_start, spp, max_depth, min_depth, seed, ANA_RENDER_CLEAR_FILM)
-        img = np.zeros((height, width, 3), np.float32)
+        img = np.empty((height, width, 3), np.float32)
         self._check(lib().ana_forward(self.h, C.byref(r), C.byref(st) if st is not None else None,
                                       img.ctypes.data))
         del keep
@@ -517,7 +517,7 @@ class Renderer:
         """IMaterial::evaluate and sample of `material` on the device for a
         BSDF_QUERY record array; returns BSDF_RESULT records."""
         q = np.ascontiguousarray(queries, BSDF_QUERY)
-        out = np.zeros(len(q), BSDF_RESULT)
+        out = np.empty(len(q), BSDF_RESULT)
         m = material_struct(material)
         self._check(lib().ana_bsdf_batch(self.h, C.byref(m), _ptr(q), len(q), _ptr(out)))
         return out
@@ -530,7 +530,7 @@ class Renderer:
     def trace(self, rays: np.ndarray, occlusion=False, times=None) -> np.ndarray:
         """ana_trace_batch (ana_trace_batch_timed with per-ray `times`)."""
         rays = np.ascontiguousarray(np.asarray(rays, np.float32).reshape(-1, 8))
-        out = np.zeros(len(rays), HIT_DTYPE)
+        out = np.empty(len(rays), HIT_DTYPE)
         if times is None:
             self._check(lib().ana_trace_batch(self.h, rays.ctypes.data, len(rays), out.ctypes.data,
                                               1 if occlusion else 0, 0))
@@ -546,7 +546,7 @@ class Renderer:
         device scratch (at most TRACE_NOALLOC_MAX_RAYS rays, no device
         allocation), for callers that must not allocate while tracing."""
         rays = np.ascontiguousarray(np.asarray(rays, np.float32).reshape(-1, 8))
-        out = np.zeros(len(rays), HIT_DTYPE)
+        out = np.empty(len(rays), HIT_DTYPE)
         self._check(lib().ana_trace_batch_noalloc(self.h, rays.ctypes.data, len(rays), out.ctypes.data,
                                                   1 if occlusion else 0))
         return out
@@ -568,7 +568,7 @@ class Renderer:
         self._check(lib().ana_render_batch(self.h, arr, len(descs), flags))
 
     def batch_film(self, item, width, height) -> np.ndarray:
-        out = np.zeros((height, width, 5), np.float32)
+        out = np.empty((height, width, 5), np.float32)
         self._check(lib().ana_batch_film_read(self.h, item, out.ctypes.data, width * height))
         return out
 

@@ -28,7 +28,8 @@ SOURCES = {
                    "traverse.cuh", "motion.cuh"],
     "build.cu": ["build.cu", "build.h", "layout.h"],
     "prepare.cpp": ["prepare.cpp", "prepare.h", "layout.h"],
-    "capi.cpp": ["capi.cpp", "kernels.h", "prepare.h", "build.h", "layout.h"],
+    "capi.cpp": ["capi.cpp", "kernels.h", "prepare.h", "build.h", "layout.h", "staging.h"],
+    "staging.cpp": ["staging.cpp", "staging.h"],
     "film_io.cpp": ["film_io.cpp"],
 }
 

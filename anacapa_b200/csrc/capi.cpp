@@ -17,6 +17,7 @@
 #include "build.h"
 #include "kernels.h"
 #include "prepare.h"
+#include "staging.h"
 
 namespace {
 
@@ -326,6 +327,14 @@ struct ana_ctx {
     size_t adj_size = 0;
     uint32_t adj_cap = 0;
     float* adj_L = nullptr;
+    // pinned words of short copies (query records, counters), pinned chunks of
+    // long ones, and the device buffers of ray queries and resolved images
+    unsigned char* pin = nullptr;
+    ana::HostStage stage;
+    unsigned char* d_query = nullptr;
+    size_t query_size = 0;
+    unsigned char* d_image = nullptr;
+    size_t image_size = 0;
     unsigned char* d_adj_io = nullptr;  // adjoint image + gradient accumulators
     size_t adj_io_size = 0;
     ana_film_pixel* film_px() const { return reinterpret_cast<ana_film_pixel*>(film); }
@@ -369,10 +378,47 @@ int ensure_buffer(ana_ctx* c, unsigned char** p, size_t* have, size_t need, cons
     }
     drop_graph(c);
     void* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, need);
+    if (e == cudaErrorMemoryAllocation && (c->d_query || c->d_image)) {  // what is only kept makes room
+        cudaGetLastError();
+        CK(cudaStreamSynchronize(c->stream), "sync");
+        cudaFree(c->d_query);
+        cudaFree(c->d_image);
+        c->d_query = c->d_image = nullptr;
+        c->query_size = c->image_size = 0;
+        e = cudaMalloc(&mem, need);
+    }
+    CK(e, what);
+    *p = static_cast<unsigned char*>(mem);
+    *have = need;
+    return ANA_OK;
+}
+
+// Pinned words of a context (ana_ctx::pin, null when none could be had).
+constexpr size_t kPinBytes = size_t(1) << 17;
+
+// Query and image buffers are kept between calls up to this size; a larger one
+// is freed when its call ends.
+constexpr size_t kKeepBytes = size_t(256) << 20;
+
+// Grows a buffer that no captured graph refers to (contents are not kept).
+// Its last call is complete: these calls wait for the stream.
+int ensure_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need, const char* what) {
+    if (*have >= need && *p) return ANA_OK;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+    void* mem = nullptr;
     CK(cudaMalloc(&mem, need), what);
     *p = static_cast<unsigned char*>(mem);
     *have = need;
     return ANA_OK;
+}
+void trim_scratch(unsigned char** p, size_t* have) {
+    if (*have <= kKeepBytes) return;
+    cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
 }
 
 // Wavefront buffers for `cap` paths.
@@ -590,8 +636,7 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
         rc = ensure_buffer(c, &c->d_adj_io, &c->adj_io_size, oGrad + std::max<size_t>(nparams, 1) * 4,
                            "cudaMalloc(adjoint image)");
         if (rc) return rc;
-        CK(cudaMemcpyAsync(c->d_adj_io, adj_image, size_t(totalPixels) * 12, cudaMemcpyHostToDevice, c->stream),
-           "adjoint image H2D");
+        CK(c->stage.write(c->d_adj_io, adj_image, size_t(totalPixels) * 12, c->stream, c->device), "adjoint image H2D");
     }
     // film: all items back to back
     rc = ensure_buffer(c, &c->film, &c->film_bytes, totalPixels * sizeof(ana_film_pixel), "cudaMalloc(film)");
@@ -865,18 +910,31 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
     }
     CK(cudaGetLastError(), "kernel launch");
     CK(cudaEventRecord(c->ev1, c->stream), "event");
-    unsigned long long hwork[4] = {0, 0, 0, 0};
-    if (count_work)
-        CK(cudaMemcpyAsync(hwork, c->d_work, sizeof(hwork), cudaMemcpyDeviceToHost, c->stream), "work D2H");
+    // work counts, gradient, error word and counters come back together, in
+    // pinned words where they fit
     c->h_counters.resize(ncountAll);
-    CK(cudaMemcpyAsync(c->h_counters.data(), counters, ncountAll * 4, cudaMemcpyDeviceToHost, c->stream),
-       "counters D2H");
-    if (backward && nparams)
-        CK(cudaMemcpyAsync(adj_grad, c->d_adj_io + oGrad, nparams * 4, cudaMemcpyDeviceToHost, c->stream),
-           "gradient D2H");
-    uint32_t herr = 0;
-    CK(cudaMemcpyAsync(&herr, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream), "err D2H");
+    const size_t gradBytes = backward ? nparams * 4 : 0, back = 32 + 32 + align_up(gradBytes) + ncountAll * 4;
+    std::vector<unsigned char> plain;
+    unsigned char* hb = c->pin;
+    if (!hb || back > kPinBytes) {
+        plain.resize(back);
+        hb = plain.data();
+    }
+    unsigned char* const hGrad = hb + 64;
+    unsigned char* const hCount = hGrad + align_up(gradBytes);
+    if (count_work)
+        CK(cudaMemcpyAsync(hb, c->d_work, 32, cudaMemcpyDeviceToHost, c->stream), "work D2H");
+    CK(cudaMemcpyAsync(hCount, counters, ncountAll * 4, cudaMemcpyDeviceToHost, c->stream), "counters D2H");
+    if (gradBytes)
+        CK(cudaMemcpyAsync(hGrad, c->d_adj_io + oGrad, gradBytes, cudaMemcpyDeviceToHost, c->stream), "gradient D2H");
+    CK(cudaMemcpyAsync(hb + 32, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream), "err D2H");
     CK(cudaStreamSynchronize(c->stream), "render sync");
+    unsigned long long hwork[4] = {0, 0, 0, 0};
+    uint32_t herr = 0;
+    if (count_work) std::memcpy(hwork, hb, sizeof(hwork));
+    std::memcpy(&herr, hb + 32, 4);
+    std::memcpy(c->h_counters.data(), hCount, ncountAll * 4);
+    if (gradBytes) std::memcpy(adj_grad, hGrad, gradBytes);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     ana_stats& st = c->stats;
@@ -1030,6 +1088,9 @@ int ana_create(ana_ctx** out, const ana_device_opts* opts) {
     cudaMemset(c->d_err, 0, 256);
     cudaEventCreate(&c->ev0);
     cudaEventCreate(&c->ev1);
+    void* pin = nullptr;
+    if (cudaHostAlloc(&pin, kPinBytes, cudaHostAllocPortable) == cudaSuccess) c->pin = static_cast<unsigned char*>(pin);
+    else cudaGetLastError();
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
     ana::prime_kernels();
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "kernel load");
@@ -1052,6 +1113,10 @@ void ana_destroy(ana_ctx* c) {
     cudaFree(c->d_err);
     cudaFree(c->d_adj);
     cudaFree(c->d_adj_io);
+    cudaFree(c->d_query);
+    cudaFree(c->d_image);
+    if (c->pin) cudaFreeHost(c->pin);
+    c->stage.release();
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -1350,8 +1415,7 @@ int ana_film_read(ana_ctx* c, ana_film_pixel* out, size_t count) {
     if (count != c->film_pixels)
         return fail(c, ANA_ERR_INVALID_ARG, "ana_film_read: count != pixels of the last render");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    CK(cudaMemcpyAsync(out, c->film, count * sizeof(ana_film_pixel), cudaMemcpyDeviceToHost, c->stream), "film D2H");
-    CK(cudaStreamSynchronize(c->stream), "film sync");
+    CK(c->stage.read(out, c->film, count * sizeof(ana_film_pixel), c->stream, c->device), "film D2H");
     return ANA_OK;
 }
 
@@ -1361,10 +1425,9 @@ int ana_batch_film_read(ana_ctx* c, uint32_t item, ana_film_pixel* out, size_t c
     if (count != c->item_film_pixels[item])
         return fail(c, ANA_ERR_INVALID_ARG, "ana_batch_film_read: count != the item's pixels");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    CK(cudaMemcpyAsync(out, c->film_px() + c->item_film_offset[item], count * sizeof(ana_film_pixel),
-                       cudaMemcpyDeviceToHost, c->stream),
+    CK(c->stage.read(out, c->film_px() + c->item_film_offset[item], count * sizeof(ana_film_pixel), c->stream,
+                     c->device),
        "film D2H");
-    CK(cudaStreamSynchronize(c->stream), "film sync");
     return ANA_OK;
 }
 
@@ -1374,18 +1437,17 @@ int ana_aov_read(ana_ctx* c, float* albedo, float* normal, size_t count) {
     if (count != c->film_pixels)
         return fail(c, ANA_ERR_INVALID_ARG, "ana_aov_read: count != pixels of the last render");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    std::vector<float> h(count * 8);
-    CK(cudaMemcpyAsync(h.data(), c->aov_film, h.size() * 4, cudaMemcpyDeviceToHost, c->stream), "AOV D2H");
-    CK(cudaStreamSynchronize(c->stream), "AOV sync");
-    for (size_t i = 0; i < count; ++i)  // PixelAccumulator::resolve
-        for (int l = 0; l < 2; ++l) {
-            float* out = l ? normal : albedo;
-            if (!out) continue;
-            const float* a = h.data() + 8 * i + 4 * l;
-            const float w = a[3];
-            const float inv = w > 0.f ? 1.f / w : 0.f;
-            for (int k = 0; k < 3; ++k) out[3 * i + k] = w > 0.f ? a[k] * inv : 0.f;
-        }
+    int rc = ensure_scratch(c, &c->d_image, &c->image_size, count * 12, "cudaMalloc(resolved image)");
+    if (rc) return rc;
+    float* const img = reinterpret_cast<float*>(c->d_image);
+    for (int l = 0; l < 2; ++l) {  // PixelAccumulator::resolve, 12 of 16 bytes per pixel and layer
+        float* out = l ? normal : albedo;
+        if (!out) continue;
+        ana::launch_aov_image(reinterpret_cast<const float*>(c->aov_film), uint32_t(count), l, img, c->stream);
+        CK(cudaGetLastError(), "AOV resolve");
+        CK(c->stage.read(out, img, count * 12, c->stream, c->device), "AOV D2H");
+    }
+    trim_scratch(&c->d_image, &c->image_size);
     return ANA_OK;
 }
 
@@ -1443,6 +1505,76 @@ int ana_film_device_ptr(ana_ctx* c, void** dptr) {
     return ANA_OK;
 }
 
+// Queries of up to this many rays cross the bus through the context's pinned
+// words, one copy each way.
+constexpr size_t kSmallQuery = 1024;
+static_assert(ana::trace_times_offset(kSmallQuery) <= kPinBytes, "small queries fit the pinned words");
+
+// A ray query against scene 0 in the device buffer `base` (kernels.h,
+// kTraceRays). Host rays and hits unless on_device; times like the rays, or
+// null. `staged`: long copies may use the context's pinned chunks (which the
+// first of them allocates).
+static cudaError_t run_query(ana_ctx* c, unsigned char* base, const float* rays, const float* times, size_t n,
+                             ana_hit* out, int occlusion, int on_device, bool staged, uint32_t& herr) {
+    ana::DevSceneRec R{};
+    R.tri_root = c->scenes[0].tri_root;
+    R.seg_root = c->scenes[0].seg_root;
+    const size_t nb = on_device ? 0 : n;  // rays in the buffer
+    unsigned char* const d_state = base + ana::trace_state_offset(nb);
+    const bool small = c->pin && !on_device && !times && n <= kSmallQuery;
+    const float* d_rays = on_device ? rays : reinterpret_cast<const float*>(base + ana::kTraceRays);
+    ana_hit* d_out = on_device ? out : reinterpret_cast<ana_hit*>(base + ana::trace_hits_offset(nb));
+    const float* d_times = times;
+    cudaError_t e = cudaSuccess;
+    if (small) {
+        std::memset(c->pin, 0, ana::kTraceRays);
+        std::memcpy(c->pin, &R, sizeof(R));
+        std::memcpy(c->pin + ana::kTraceRays, rays, n * 32);
+        std::memset(c->pin + ana::trace_state_offset(n), 0, ana::kTraceState);
+        e = cudaMemcpyAsync(base, c->pin, ana::trace_hits_offset(n), cudaMemcpyHostToDevice, c->stream);
+    } else {
+        e = cudaMemcpyAsync(base, &R, sizeof(R), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(d_state, 0, ana::kTraceState, c->stream);
+        auto put = [&](void* dst, const void* src, size_t bytes) {
+            return staged ? c->stage.write(dst, src, bytes, c->stream, c->device)
+                          : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
+        };
+        if (!on_device) {
+            if (e == cudaSuccess) e = put(base + ana::kTraceRays, rays, n * 32);
+            if (times) {
+                unsigned char* const t = base + ana::trace_times_offset(n);
+                if (e == cudaSuccess) e = put(t, times, n * 4);
+                d_times = reinterpret_cast<const float*>(t);
+            }
+        }
+    }
+    if (e != cudaSuccess) return e;
+    ana::DevScene S = c->ds;
+    S.scenes = reinterpret_cast<const ana::DevSceneRec*>(base);
+    S.num_scenes = 1;
+    uint32_t* const state = reinterpret_cast<uint32_t*>(d_state);
+    ana::launch_trace_batch(S, 0, d_rays, d_times, n, d_out, occlusion, state + 1, state,
+                            c->opts.traversal == ANA_TRAVERSAL_PER_RAY ? 0 : 1, c->stream);
+    e = cudaGetLastError();
+    if (small) {
+        unsigned char* const h = c->pin + ana::trace_state_offset(n);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h, d_state, ana::kTraceState + n * 32, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e == cudaSuccess) {
+            std::memcpy(&herr, h, 4);
+            std::memcpy(out, h + ana::kTraceState, n * 32);
+        }
+        return e;
+    }
+    if (e == cudaSuccess && !on_device)
+        e = staged ? c->stage.read(out, d_out, n * sizeof(ana_hit), c->stream, c->device)
+                   : cudaMemcpyAsync(out, d_out, n * sizeof(ana_hit), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, d_state, 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    return e;
+}
+
 // ana_trace_batch with optional per-ray times (host or device like the rays).
 static int trace_batch(ana_ctx* c, const float* rays, const float* times, size_t n, ana_hit* out, int occlusion,
                        int on_device) {
@@ -1451,48 +1583,12 @@ static int trace_batch(ana_ctx* c, const float* rays, const float* times, size_t
     if (n == 0) return ANA_OK;
     if (n >= (size_t(1) << 32) - 64) return fail(c, ANA_ERR_INVALID_ARG, "ana_trace_batch: n >= 2^32");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    // one scene record (scene 0: its roots) ahead of the rays
-    ana::DevSceneRec R{};
-    R.tri_root = c->scenes[0].tri_root;
-    R.seg_root = c->scenes[0].seg_root;
-    const size_t recBytes = align_up(sizeof(R));
-    const size_t tmpBytes = recBytes + (on_device ? 0 : n * 32 + n * sizeof(ana_hit) + (times ? n * 4 : 0));
-    void* tmp = nullptr;
-    CK(cudaMalloc(&tmp, tmpBytes), "cudaMalloc(trace batch)");
-    unsigned char* tb = static_cast<unsigned char*>(tmp);
-    const float* d_rays = rays;
-    const float* d_times = times;
-    ana_hit* d_out = out;
-    cudaError_t e = cudaMemcpyAsync(tb, &R, sizeof(R), cudaMemcpyHostToDevice, c->stream);
-    if (!on_device) {
-        d_rays = reinterpret_cast<const float*>(tb + recBytes);
-        d_out = reinterpret_cast<ana_hit*>(tb + recBytes + n * 32);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(tb + recBytes, rays, n * 32, cudaMemcpyHostToDevice, c->stream);
-        if (times) {
-            float* t = reinterpret_cast<float*>(tb + recBytes + n * 32 + n * sizeof(ana_hit));
-            d_times = t;
-            if (e == cudaSuccess) e = cudaMemcpyAsync(t, times, n * 4, cudaMemcpyHostToDevice, c->stream);
-        }
-    }
-    uint32_t* d_fetch = c->d_err + 32;  // fetch counter of the persistent kernel
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_err, 0, 4, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_fetch, 0, 4, c->stream);
-    if (e != cudaSuccess) {
-        cudaFree(tmp);
-        return cuda_fail(c, e, "trace batch setup");
-    }
-    ana::DevScene S = c->ds;
-    S.scenes = reinterpret_cast<const ana::DevSceneRec*>(tb);
-    S.num_scenes = 1;
-    ana::launch_trace_batch(S, 0, d_rays, d_times, n, d_out, occlusion, d_fetch, c->d_err,
-                            c->opts.traversal == ANA_TRAVERSAL_PER_RAY ? 0 : 1, c->stream);
-    e = cudaGetLastError();
+    const size_t bytes = on_device ? ana::trace_hits_offset(0) : ana::trace_times_offset(n) + (times ? n * 4 : 0);
+    const int rc = ensure_scratch(c, &c->d_query, &c->query_size, bytes, "cudaMalloc(trace batch)");
+    if (rc) return rc;
     uint32_t herr = 0;
-    if (e == cudaSuccess && !on_device)
-        e = cudaMemcpyAsync(out, d_out, n * sizeof(ana_hit), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
+    const cudaError_t e = run_query(c, c->d_query, rays, times, n, out, occlusion, on_device, true, herr);
+    trim_scratch(&c->d_query, &c->query_size);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace batch");
     if (herr) return fail(c, ANA_ERR_DEVICE_CHECK, "ana_trace_batch: traversal stack overflow on the device");
     return ANA_OK;
@@ -1508,9 +1604,8 @@ int ana_trace_batch_timed(ana_ctx* c, const float* rays, const float* times, siz
 }
 
 // The same query as ana_trace_batch with host buffers, staged in the fixed
-// module scratch (kernels.cu) instead of a per-call cudaMalloc: callers that
-// must not allocate (a pick query beside an in-flight frame, where cudaFree
-// would wait for the frame; a device already full) use this one. Nothing on
+// module scratch (kernels.cu): callers that must not allocate (a pick query
+// beside an in-flight frame; a device already full) use this one. Nothing on
 // the success path allocates, on the device or on the host.
 int ana_trace_batch_noalloc(ana_ctx* c, const float* rays, size_t n, ana_hit* out, int occlusion) {
     if (!c || (!rays && n) || (!out && n))
@@ -1526,28 +1621,8 @@ int ana_trace_batch_noalloc(ana_ctx* c, const float* rays, size_t n, ana_hit* ou
     unsigned char* base = nullptr;
     cudaError_t e = ana::noalloc_trace_scratch(c->device, &base);
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_trace_batch_noalloc: scratch address (cudaGetSymbolAddress)");
-    ana::DevSceneRec R{};
-    R.tri_root = c->scenes[0].tri_root;
-    R.seg_root = c->scenes[0].seg_root;
-    float* d_rays = reinterpret_cast<float*>(base + ana::kNoAllocRays);
-    ana_hit* d_out = reinterpret_cast<ana_hit*>(base + ana::kNoAllocHits);
-    uint32_t* d_err = reinterpret_cast<uint32_t*>(base + ana::kNoAllocErrOffset);
-    uint32_t* d_fetch = d_err + 1;
-    e = cudaMemcpyAsync(base, &R, sizeof(R), cudaMemcpyHostToDevice, c->stream);
-    // the error word and the persistent schedule's work counter start at zero
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_err, 0, 8, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_rays, rays, n * 32, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "ana_trace_batch_noalloc: setup");
-    ana::DevScene S = c->ds;
-    S.scenes = reinterpret_cast<const ana::DevSceneRec*>(base);
-    S.num_scenes = 1;
-    ana::launch_trace_batch(S, 0, d_rays, nullptr, n, d_out, occlusion, d_fetch, d_err,
-                            c->opts.traversal == ANA_TRAVERSAL_PER_RAY ? 0 : 1, c->stream);
-    e = cudaGetLastError();
     uint32_t herr = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, n * sizeof(ana_hit), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, d_err, 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    e = run_query(c, base, rays, nullptr, n, out, occlusion, 0, false, herr);
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_trace_batch_noalloc");
     if (herr) return fail(c, ANA_ERR_DEVICE_CHECK, "ana_trace_batch_noalloc: traversal stack overflow on the device");
     return ANA_OK;
@@ -1564,18 +1639,18 @@ int ana_bsdf_batch(ana_ctx* c, const ana_material* material, const ana_bsdf_quer
     if (n == 0) return ANA_OK;
     CK(cudaSetDevice(c->device), "cudaSetDevice");
     const size_t qBytes = align_up(n * sizeof(ana_bsdf_query));
-    void* tmp = nullptr;
-    CK(cudaMalloc(&tmp, qBytes + n * sizeof(ana_bsdf_result)), "cudaMalloc(bsdf query)");
-    auto* dq = static_cast<ana_bsdf_query*>(tmp);
-    auto* dr = reinterpret_cast<ana_bsdf_result*>(static_cast<unsigned char*>(tmp) + qBytes);
-    cudaError_t e = cudaMemcpyAsync(dq, q, n * sizeof(ana_bsdf_query), cudaMemcpyHostToDevice, c->stream);
+    const int rc = ensure_scratch(c, &c->d_query, &c->query_size, qBytes + n * sizeof(ana_bsdf_result),
+                                  "cudaMalloc(bsdf query)");
+    if (rc) return rc;
+    auto* dq = reinterpret_cast<ana_bsdf_query*>(c->d_query);
+    auto* dr = reinterpret_cast<ana_bsdf_result*>(c->d_query + qBytes);
+    cudaError_t e = c->stage.write(dq, q, n * sizeof(ana_bsdf_query), c->stream, c->device);
     if (e == cudaSuccess) {
         ana::launch_bsdf_query(m, dq, uint32_t(n), dr, c->stream);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, dr, n * sizeof(ana_bsdf_result), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
+    if (e == cudaSuccess) e = c->stage.read(out, dr, n * sizeof(ana_bsdf_result), c->stream, c->device);
+    trim_scratch(&c->d_query, &c->query_size);
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_bsdf_batch");
     return ANA_OK;
 }
@@ -1643,14 +1718,12 @@ int ana_forward(ana_ctx* c, const ana_render_desc* d, const ana_diff_params* par
     c->fwd_valid = true;
     if (image) {
         const size_t n = size_t(d->width) * d->height;
-        std::vector<ana_film_pixel> px(n);
-        CK(cudaMemcpy(px.data(), c->film, n * sizeof(ana_film_pixel), cudaMemcpyDeviceToHost), "film D2H");
-        for (size_t i = 0; i < n; ++i) {  // Film::getPixel
-            const float w = px[i].w;
-            image[3 * i] = w > 0.f ? px[i].r / w : 0.f;
-            image[3 * i + 1] = w > 0.f ? px[i].g / w : 0.f;
-            image[3 * i + 2] = w > 0.f ? px[i].b / w : 0.f;
-        }
+        rc = ensure_scratch(c, &c->d_image, &c->image_size, n * 12, "cudaMalloc(resolved image)");
+        if (rc) return rc;
+        ana::launch_film_image(c->film_px(), uint32_t(n), reinterpret_cast<float*>(c->d_image), c->stream);
+        CK(cudaGetLastError(), "film resolve");
+        CK(c->stage.read(image, c->d_image, n * 12, c->stream, c->device), "image D2H");
+        trim_scratch(&c->d_image, &c->image_size);
     }
     return ANA_OK;
 }

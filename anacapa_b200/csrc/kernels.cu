@@ -1082,6 +1082,29 @@ __global__ void __launch_bounds__(256) k_film(const __grid_constant__ Params p) 
     }
 }
 
+// Resolved images for reads by the host: 12 of the film's 20 bytes and of an AOV
+// layer's 16 cross the bus, and no host loop divides (1280x720 AOVs: 11 ms on
+// the host).
+__global__ void __launch_bounds__(256) k_film_image(const ana_film_pixel* film, uint32_t n, float* out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const ana_film_pixel p = film[i];
+        const bool ok = p.w > 0.f;
+        out[3 * size_t(i)] = ok ? xdiv(p.r, p.w) : 0.f;
+        out[3 * size_t(i) + 1] = ok ? xdiv(p.g, p.w) : 0.f;
+        out[3 * size_t(i) + 2] = ok ? xdiv(p.b, p.w) : 0.f;
+    }
+}
+__global__ void __launch_bounds__(256) k_aov_image(const float4* aov, uint32_t n, int layer, float* out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 a = aov[2 * size_t(i) + layer];
+        const bool ok = a.w > 0.f;
+        const float inv = ok ? xdiv(1.f, a.w) : 0.f;
+        out[3 * size_t(i)] = ok ? xmul(a.x, inv) : 0.f;
+        out[3 * size_t(i) + 1] = ok ? xmul(a.y, inv) : 0.f;
+        out[3 * size_t(i) + 2] = ok ? xmul(a.z, inv) : 0.f;
+    }
+}
+
 // IAccelerationStructure::traceBatch / occludedBatch over CurveBrute semantics,
 // against one scene of the batch.
 template <bool kAny, bool kCurves, bool kPersist, bool kMotion = false>
@@ -1187,6 +1210,8 @@ void prime_kernels() {
     prime(k_film);
     prime(k_adj_init);
     prime(k_adj_direct);
+    prime(k_film_image);
+    prime(k_aov_image);
     prime(k_extend<false, false, false>);
     prime(k_extend<false, false, true>);
     prime(k_extend<false, true, false>);
@@ -1377,11 +1402,18 @@ void launch_adj_direct(const Params& p, const LaunchCfg& c, cudaStream_t s) {
 void launch_film(const Params& p, const LaunchCfg& c, cudaStream_t s) {
     k_film<<<blocks_for(p.chunk_pixels, 256, c.grid_cap), 256, 0, s>>>(p);
 }
+void launch_film_image(const ana_film_pixel* film, uint32_t n, float* out, cudaStream_t s) {
+    k_film_image<<<blocks_for(n, 256, 1 << 20), 256, 0, s>>>(film, n, out);
+}
+void launch_aov_image(const float* aov, uint32_t n, int layer, float* out, cudaStream_t s) {
+    k_aov_image<<<blocks_for(n, 256, 1 << 20), 256, 0, s>>>(reinterpret_cast<const float4*>(aov), n, layer, out);
+}
 template <bool kAny, bool kCurves, bool kPersist, bool kMotion = false>
 static void tb_launch(const DevScene& S, uint32_t scene, const float* rays, const float* times, uint32_t n,
                       ana_hit* out, uint32_t* fetch, uint32_t* err, int grid, cudaStream_t s) {
     auto k = k_trace_batch<kAny, kCurves, kPersist, kMotion>;
-    int g = kPersist ? resident_grid(k) : grid;
+    // a short query has no ray for the other blocks' warps (one ray each)
+    const int g = kPersist ? std::min(resident_grid(k), blocks_for(n, kPersistBlock / 32, 1 << 20)) : grid;
     k<<<g, kPersistBlock, 0, s>>>(S, scene, rays, times, n, out, fetch, err);
 }
 void launch_trace_batch(const DevScene& S, uint32_t scene, const float* rays, const float* times, size_t n,

@@ -130,21 +130,31 @@ void launch_adj_direct(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_trace_batch(const DevScene& S, uint32_t scene, const float* rays, const float* times, size_t n,
                         ana_hit* out, int occlusion, uint32_t* fetch, uint32_t* err, int persistent, cudaStream_t s);
 
+// Resolved images, 3 floats per pixel: the film's r, g, b over its weight
+// (Film::getPixel, black without weight), and one layer of the AOV film (0
+// albedo, 1 normal) times the reciprocal of its weight (PixelAccumulator::resolve).
+void launch_film_image(const ana_film_pixel* film, uint32_t n, float* out, cudaStream_t s);
+void launch_aov_image(const float* aov, uint32_t n, int layer, float* out, cudaStream_t s);
+
 // IMaterial::evaluate / sample of one material over n queries (ana_bsdf_batch).
 void launch_bsdf_query(const DevMaterial& m, const ana_bsdf_query* q, uint32_t n, ana_bsdf_result* out,
                        cudaStream_t s);
 
-// Fixed device scratch of the allocation-free trace entry point: a 256-byte
-// header (the scene record at 0, the error word at kNoAllocErrOffset and the
-// persistent schedule's work counter 4 bytes after it), then room for
-// ANA_TRACE_NOALLOC_MAX_RAYS rays of 32 bytes, then as many 32-byte hits.
-constexpr size_t kNoAllocHeader = 256;
-constexpr size_t kNoAllocErrOffset = 240;
-constexpr size_t kNoAllocRays = kNoAllocHeader;
-constexpr size_t kNoAllocHits = kNoAllocRays + size_t(ANA_TRACE_NOALLOC_MAX_RAYS) * 32;
-constexpr size_t kNoAllocBytes = kNoAllocHits + size_t(ANA_TRACE_NOALLOC_MAX_RAYS) * sizeof(ana_hit);
-static_assert(sizeof(DevSceneRec) <= kNoAllocErrOffset, "scene record overlaps the error word");
+// Device buffer of a ray query: the scene record, the rays (32 bytes each), a
+// state block (error word, then the persistent schedule's work counter), the
+// hits (32 bytes each), and the ray times if any. What goes to the device (up
+// to the state block) and what comes back (from it) are contiguous, one copy
+// each for a small query.
+constexpr size_t kTraceRays = 256, kTraceState = 32;
+constexpr size_t trace_state_offset(size_t n) { return kTraceRays + 32 * n; }
+constexpr size_t trace_hits_offset(size_t n) { return trace_state_offset(n) + kTraceState; }
+constexpr size_t trace_times_offset(size_t n) { return trace_hits_offset(n) + 32 * n; }
+static_assert(sizeof(DevSceneRec) <= kTraceRays, "scene record overlaps the rays");
 static_assert(sizeof(ana_hit) == 32, "hit record size");
+
+// Fixed device scratch of the allocation-free trace entry point: that buffer
+// for ANA_TRACE_NOALLOC_MAX_RAYS rays without times.
+constexpr size_t kNoAllocBytes = trace_times_offset(ANA_TRACE_NOALLOC_MAX_RAYS);
 
 // Device address of that scratch on `device`, which must be the current
 // device. The first call per device looks it up (cudaGetSymbolAddress) and

@@ -1,0 +1,112 @@
+#include "staging.h"
+
+#include <algorithm>
+#include <cstring>
+#include <system_error>
+#include <thread>
+
+namespace ana {
+
+// Copies below this take the driver's path: the threads cost more than they
+// save (0.1-0.2 ms for starting and joining them).
+static constexpr size_t kStageMin = size_t(1) << 20;
+
+void HostStage::release() {
+    for (int t = 0; t < kThreads; ++t) {
+        if (stream_[t]) cudaStreamDestroy(stream_[t]);
+        stream_[t] = nullptr;
+        for (cudaEvent_t& e : done_[t]) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+    }
+    if (begin_) cudaEventDestroy(begin_);
+    begin_ = nullptr;
+    if (pinned_) cudaFreeHost(pinned_);
+    pinned_ = nullptr;
+}
+
+bool HostStage::ensure() {
+    if (pinned_) return true;
+    if (failed_) return false;
+    void* p = nullptr;
+    bool ok = cudaHostAlloc(&p, kThreads * 2 * kChunk, cudaHostAllocPortable) == cudaSuccess;
+    if (ok) pinned_ = static_cast<unsigned char*>(p);
+    ok = ok && cudaEventCreateWithFlags(&begin_, cudaEventDisableTiming) == cudaSuccess;
+    for (int t = 0; ok && t < kThreads; ++t) {
+        ok = cudaStreamCreateWithFlags(&stream_[t], cudaStreamNonBlocking) == cudaSuccess;
+        for (cudaEvent_t& e : done_[t]) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (!ok) {  // no pinned memory to be had: the driver's path from now on
+        cudaGetLastError();
+        release();
+        failed_ = true;
+    }
+    return ok;
+}
+
+// Thread t's chunks t, t + threads, ...
+cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, int device,
+                           bool out) {
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_[t], begin_, 0);
+    const size_t chunks = (bytes + kChunk - 1) / kChunk, step = size_t(threads);
+    unsigned char* slot[2] = {pinned_ + size_t(2 * t) * kChunk, pinned_ + size_t(2 * t + 1) * kChunk};
+    auto size_of = [&](size_t k) { return std::min(kChunk, bytes - k * kChunk); };
+    auto fetch = [&](size_t k, int s) {
+        cudaError_t r = cudaMemcpyAsync(slot[s], src + k * kChunk, size_of(k), cudaMemcpyDeviceToHost, stream_[t]);
+        return r == cudaSuccess ? cudaEventRecord(done_[t][s], stream_[t]) : r;
+    };
+    int s = 0;
+    if (out) {
+        if (e == cudaSuccess && size_t(t) < chunks) e = fetch(size_t(t), 0);
+        for (size_t k = size_t(t); e == cudaSuccess && k < chunks; k += step, s ^= 1) {
+            if (k + step < chunks) e = fetch(k + step, s ^ 1);
+            if (e == cudaSuccess) e = cudaEventSynchronize(done_[t][s]);
+            if (e == cudaSuccess) std::memcpy(dst + k * kChunk, slot[s], size_of(k));
+        }
+    } else {
+        for (size_t k = size_t(t), i = 0; e == cudaSuccess && k < chunks; k += step, ++i, s ^= 1) {
+            if (i >= 2) e = cudaEventSynchronize(done_[t][s]);  // the slot's last copy has left it
+            if (e != cudaSuccess) break;
+            std::memcpy(slot[s], src + k * kChunk, size_of(k));
+            e = cudaMemcpyAsync(dst + k * kChunk, slot[s], size_of(k), cudaMemcpyHostToDevice, stream_[t]);
+            if (e == cudaSuccess) e = cudaEventRecord(done_[t][s], stream_[t]);
+        }
+    }
+    const cudaError_t f = cudaStreamSynchronize(stream_[t]);  // the slots are free for the next copy
+    return e == cudaSuccess ? f : e;
+}
+
+// 1920x1080 film (41 MB) into fresh pages 4.9 -> 2.4 ms (1.8 into used ones, 23
+// GB/s), 960x540 film (10 MB) into used pages 0.38; 2^20 rays in and hits out (32
+// MB each) with their traversal 7.5 -> 4.6 ms.
+cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream_t st, int device, bool out) {
+    if (bytes < kStageMin || !ensure()) {
+        cudaError_t e = cudaMemcpyAsync(dst, src, bytes, out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && out) e = cudaStreamSynchronize(st);
+        return e;
+    }
+    cudaError_t e = cudaEventRecord(begin_, st);
+    if (e != cudaSuccess) return e;
+    const unsigned cores = std::thread::hardware_concurrency();
+    const int threads = int(std::min<size_t>({size_t(kThreads), std::max<size_t>(1, cores / 2), (bytes + kChunk - 1) / kChunk}));
+    cudaError_t result[kThreads] = {};
+    auto work = [&](int t) {
+        result[t] = run(t, threads, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, device, out);
+    };
+    std::thread pool[kThreads];
+    int started = 1;
+    try {
+        for (; started < threads; ++started) pool[started] = std::thread(work, started);
+    } catch (const std::system_error&) {  // no more threads to be had: this one does their part
+    }
+    work(0);
+    for (int t = started; t < threads; ++t) work(t);
+    for (int t = 1; t < started; ++t) pool[t].join();
+    for (int t = 0; t < threads; ++t)
+        if (result[t] != cudaSuccess) e = result[t];
+    return e;
+}
+
+}  // namespace ana
