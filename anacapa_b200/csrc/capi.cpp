@@ -327,10 +327,9 @@ struct ana_ctx {
     size_t adj_size = 0;
     uint32_t adj_cap = 0;
     float* adj_L = nullptr;
-    // pinned words of short copies (query records, counters), pinned chunks of
-    // long ones, and the device buffers of ray queries and resolved images
+    // pinned words of short copies (query records, counters), and the device
+    // buffers of ray queries and resolved images
     unsigned char* pin = nullptr;
-    ana::HostStage stage;
     unsigned char* d_query = nullptr;
     size_t query_size = 0;
     unsigned char* d_image = nullptr;
@@ -636,7 +635,7 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
         rc = ensure_buffer(c, &c->d_adj_io, &c->adj_io_size, oGrad + std::max<size_t>(nparams, 1) * 4,
                            "cudaMalloc(adjoint image)");
         if (rc) return rc;
-        CK(c->stage.write(c->d_adj_io, adj_image, size_t(totalPixels) * 12, c->stream, c->device), "adjoint image H2D");
+        CK(ana::stage_write(c->d_adj_io, adj_image, size_t(totalPixels) * 12, c->stream, c->device), "adjoint image H2D");
     }
     // film: all items back to back
     rc = ensure_buffer(c, &c->film, &c->film_bytes, totalPixels * sizeof(ana_film_pixel), "cudaMalloc(film)");
@@ -1094,6 +1093,7 @@ int ana_create(ana_ctx** out, const ana_device_opts* opts) {
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
     ana::prime_kernels();
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "kernel load");
+    ana::stage_retain();
     *out = c;
     return ANA_OK;
 }
@@ -1116,7 +1116,7 @@ void ana_destroy(ana_ctx* c) {
     cudaFree(c->d_query);
     cudaFree(c->d_image);
     if (c->pin) cudaFreeHost(c->pin);
-    c->stage.release();
+    ana::stage_release();
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -1415,7 +1415,7 @@ int ana_film_read(ana_ctx* c, ana_film_pixel* out, size_t count) {
     if (count != c->film_pixels)
         return fail(c, ANA_ERR_INVALID_ARG, "ana_film_read: count != pixels of the last render");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    CK(c->stage.read(out, c->film, count * sizeof(ana_film_pixel), c->stream, c->device), "film D2H");
+    CK(ana::stage_read(out, c->film, count * sizeof(ana_film_pixel), c->stream, c->device), "film D2H");
     return ANA_OK;
 }
 
@@ -1425,7 +1425,7 @@ int ana_batch_film_read(ana_ctx* c, uint32_t item, ana_film_pixel* out, size_t c
     if (count != c->item_film_pixels[item])
         return fail(c, ANA_ERR_INVALID_ARG, "ana_batch_film_read: count != the item's pixels");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    CK(c->stage.read(out, c->film_px() + c->item_film_offset[item], count * sizeof(ana_film_pixel), c->stream,
+    CK(ana::stage_read(out, c->film_px() + c->item_film_offset[item], count * sizeof(ana_film_pixel), c->stream,
                      c->device),
        "film D2H");
     return ANA_OK;
@@ -1445,7 +1445,7 @@ int ana_aov_read(ana_ctx* c, float* albedo, float* normal, size_t count) {
         if (!out) continue;
         ana::launch_aov_image(reinterpret_cast<const float*>(c->aov_film), uint32_t(count), l, img, c->stream);
         CK(cudaGetLastError(), "AOV resolve");
-        CK(c->stage.read(out, img, count * 12, c->stream, c->device), "AOV D2H");
+        CK(ana::stage_read(out, img, count * 12, c->stream, c->device), "AOV D2H");
     }
     trim_scratch(&c->d_image, &c->image_size);
     return ANA_OK;
@@ -1512,7 +1512,7 @@ static_assert(ana::trace_times_offset(kSmallQuery) <= kPinBytes, "small queries 
 
 // A ray query against scene 0 in the device buffer `base` (kernels.h,
 // kTraceRays). Host rays and hits unless on_device; times like the rays, or
-// null. `staged`: long copies may use the context's pinned chunks (which the
+// null. `staged`: long copies may use the shared pinned chunks (which the
 // first of them allocates).
 static cudaError_t run_query(ana_ctx* c, unsigned char* base, const float* rays, const float* times, size_t n,
                              ana_hit* out, int occlusion, int on_device, bool staged, uint32_t& herr) {
@@ -1536,7 +1536,7 @@ static cudaError_t run_query(ana_ctx* c, unsigned char* base, const float* rays,
         e = cudaMemcpyAsync(base, &R, sizeof(R), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(d_state, 0, ana::kTraceState, c->stream);
         auto put = [&](void* dst, const void* src, size_t bytes) {
-            return staged ? c->stage.write(dst, src, bytes, c->stream, c->device)
+            return staged ? ana::stage_write(dst, src, bytes, c->stream, c->device)
                           : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
         };
         if (!on_device) {
@@ -1568,7 +1568,7 @@ static cudaError_t run_query(ana_ctx* c, unsigned char* base, const float* rays,
         return e;
     }
     if (e == cudaSuccess && !on_device)
-        e = staged ? c->stage.read(out, d_out, n * sizeof(ana_hit), c->stream, c->device)
+        e = staged ? ana::stage_read(out, d_out, n * sizeof(ana_hit), c->stream, c->device)
                    : cudaMemcpyAsync(out, d_out, n * sizeof(ana_hit), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, d_state, 4, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1644,12 +1644,12 @@ int ana_bsdf_batch(ana_ctx* c, const ana_material* material, const ana_bsdf_quer
     if (rc) return rc;
     auto* dq = reinterpret_cast<ana_bsdf_query*>(c->d_query);
     auto* dr = reinterpret_cast<ana_bsdf_result*>(c->d_query + qBytes);
-    cudaError_t e = c->stage.write(dq, q, n * sizeof(ana_bsdf_query), c->stream, c->device);
+    cudaError_t e = ana::stage_write(dq, q, n * sizeof(ana_bsdf_query), c->stream, c->device);
     if (e == cudaSuccess) {
         ana::launch_bsdf_query(m, dq, uint32_t(n), dr, c->stream);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = c->stage.read(out, dr, n * sizeof(ana_bsdf_result), c->stream, c->device);
+    if (e == cudaSuccess) e = ana::stage_read(out, dr, n * sizeof(ana_bsdf_result), c->stream, c->device);
     trim_scratch(&c->d_query, &c->query_size);
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_bsdf_batch");
     return ANA_OK;
@@ -1722,7 +1722,7 @@ int ana_forward(ana_ctx* c, const ana_render_desc* d, const ana_diff_params* par
         if (rc) return rc;
         ana::launch_film_image(c->film_px(), uint32_t(n), reinterpret_cast<float*>(c->d_image), c->stream);
         CK(cudaGetLastError(), "film resolve");
-        CK(c->stage.read(image, c->d_image, n * 12, c->stream, c->device), "image D2H");
+        CK(ana::stage_read(image, c->d_image, n * 12, c->stream, c->device), "image D2H");
         trim_scratch(&c->d_image, &c->image_size);
     }
     return ANA_OK;

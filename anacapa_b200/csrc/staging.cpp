@@ -2,33 +2,53 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
+#include <mutex>
+#include <new>
 #include <system_error>
 #include <thread>
+#include <vector>
 
 namespace ana {
 
+namespace {
+
+class HostStage {
+public:
+    explicit HostStage(int device) : device_(device) {}
+    ~HostStage();
+    HostStage(const HostStage&) = delete;
+    HostStage& operator=(const HostStage&) = delete;
+    int device() const { return device_; }
+    bool make();  // on the current device; false: no pinned memory to be had
+    cudaError_t copy(void* dst, const void* src, size_t bytes, cudaStream_t st, bool out);
+
+private:
+    static constexpr int kThreads = 4;
+    static constexpr size_t kChunk = size_t(1) << 20;
+    cudaError_t run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, bool out);
+    int device_;
+    unsigned char* pinned_ = nullptr;
+    cudaStream_t stream_[kThreads] = {};
+    cudaEvent_t done_[kThreads][2] = {};
+    cudaEvent_t begin_ = nullptr;
+};
+
 // Copies below this take the driver's path: the threads cost more than they
 // save (0.1-0.2 ms for starting and joining them).
-static constexpr size_t kStageMin = size_t(1) << 20;
+constexpr size_t kStageMin = size_t(1) << 20;
 
-void HostStage::release() {
+HostStage::~HostStage() {
     for (int t = 0; t < kThreads; ++t) {
         if (stream_[t]) cudaStreamDestroy(stream_[t]);
-        stream_[t] = nullptr;
-        for (cudaEvent_t& e : done_[t]) {
+        for (cudaEvent_t e : done_[t])
             if (e) cudaEventDestroy(e);
-            e = nullptr;
-        }
     }
     if (begin_) cudaEventDestroy(begin_);
-    begin_ = nullptr;
     if (pinned_) cudaFreeHost(pinned_);
-    pinned_ = nullptr;
 }
 
-bool HostStage::ensure() {
-    if (pinned_) return true;
-    if (failed_) return false;
+bool HostStage::make() {
     void* p = nullptr;
     bool ok = cudaHostAlloc(&p, kThreads * 2 * kChunk, cudaHostAllocPortable) == cudaSuccess;
     if (ok) pinned_ = static_cast<unsigned char*>(p);
@@ -37,18 +57,13 @@ bool HostStage::ensure() {
         ok = cudaStreamCreateWithFlags(&stream_[t], cudaStreamNonBlocking) == cudaSuccess;
         for (cudaEvent_t& e : done_[t]) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     }
-    if (!ok) {  // no pinned memory to be had: the driver's path from now on
-        cudaGetLastError();
-        release();
-        failed_ = true;
-    }
+    if (!ok) cudaGetLastError();
     return ok;
 }
 
 // Thread t's chunks t, t + threads, ...
-cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, int device,
-                           bool out) {
-    cudaError_t e = cudaSetDevice(device);
+cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, bool out) {
+    cudaError_t e = cudaSetDevice(device_);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_[t], begin_, 0);
     const size_t chunks = (bytes + kChunk - 1) / kChunk, step = size_t(threads);
     unsigned char* slot[2] = {pinned_ + size_t(2 * t) * kChunk, pinned_ + size_t(2 * t + 1) * kChunk};
@@ -81,19 +96,14 @@ cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigne
 // 1920x1080 film (41 MB) into fresh pages 4.9 -> 2.4 ms (1.8 into used ones, 23
 // GB/s), 960x540 film (10 MB) into used pages 0.38; 2^20 rays in and hits out (32
 // MB each) with their traversal 7.5 -> 4.6 ms.
-cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream_t st, int device, bool out) {
-    if (bytes < kStageMin || !ensure()) {
-        cudaError_t e = cudaMemcpyAsync(dst, src, bytes, out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess && out) e = cudaStreamSynchronize(st);
-        return e;
-    }
+cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream_t st, bool out) {
     cudaError_t e = cudaEventRecord(begin_, st);
     if (e != cudaSuccess) return e;
     const unsigned cores = std::thread::hardware_concurrency();
     const int threads = int(std::min<size_t>({size_t(kThreads), std::max<size_t>(1, cores / 2), (bytes + kChunk - 1) / kChunk}));
     cudaError_t result[kThreads] = {};
     auto work = [&](int t) {
-        result[t] = run(t, threads, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, device, out);
+        result[t] = run(t, threads, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, out);
     };
     std::thread pool[kThreads];
     int started = 1;
@@ -107,6 +117,73 @@ cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream
     for (int t = 0; t < threads; ++t)
         if (result[t] != cudaSuccess) e = result[t];
     return e;
+}
+
+// The sets not in use. Never destroyed itself: at the process's end the driver
+// may be gone before it.
+struct Pool {
+    std::mutex mu;
+    int contexts = 0;
+    std::vector<std::unique_ptr<HostStage>> idle;
+};
+Pool& pool() {
+    static Pool* p = new Pool;
+    return *p;
+}
+constexpr size_t kIdle = 2;
+
+std::unique_ptr<HostStage> take(int device) {
+    {
+        std::lock_guard<std::mutex> lk(pool().mu);
+        auto& idle = pool().idle;
+        for (size_t i = 0; i < idle.size(); ++i)
+            if (idle[i]->device() == device) {
+                std::unique_ptr<HostStage> s = std::move(idle[i]);
+                idle.erase(idle.begin() + std::ptrdiff_t(i));
+                return s;
+            }
+    }
+    std::unique_ptr<HostStage> s(new (std::nothrow) HostStage(device));
+    if (s && !s->make()) s.reset();
+    return s;
+}
+
+void give_back(std::unique_ptr<HostStage> s) {
+    std::lock_guard<std::mutex> lk(pool().mu);
+    if (pool().contexts > 0 && pool().idle.size() < kIdle) pool().idle.push_back(std::move(s));
+    // else freed here
+}
+
+cudaError_t staged(void* dst, const void* src, size_t bytes, cudaStream_t st, int device, bool out) {
+    if (bytes >= kStageMin) {
+        if (std::unique_ptr<HostStage> s = take(device)) {
+            const cudaError_t e = s->copy(dst, src, bytes, st, out);
+            if (e == cudaSuccess) give_back(std::move(s));  // after an error its events say nothing: freed
+            return e;
+        }
+    }
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && out) e = cudaStreamSynchronize(st);
+    return e;
+}
+
+}  // namespace
+
+void stage_retain() {
+    std::lock_guard<std::mutex> lk(pool().mu);
+    pool().contexts++;
+}
+void stage_release() {
+    std::vector<std::unique_ptr<HostStage>> gone;
+    std::lock_guard<std::mutex> lk(pool().mu);
+    if (--pool().contexts == 0) gone.swap(pool().idle);
+}
+
+cudaError_t stage_read(void* dst, const void* src, size_t bytes, cudaStream_t st, int device) {
+    return staged(dst, src, bytes, st, device, true);
+}
+cudaError_t stage_write(void* dst, const void* src, size_t bytes, cudaStream_t st, int device) {
+    return staged(dst, src, bytes, st, device, false);
 }
 
 }  // namespace ana
