@@ -284,7 +284,7 @@ __device__ __forceinline__ void run_traversal(const DevScene& S, uint32_t n, uin
 // Persistent triangle kernels fit 5 blocks per SM at 48 registers without
 // spills (1920x1080x64 throughput frame: 290.2 ms; 293.8 at 56 registers and
 // 36 warps per SM, 292.2 at 40 and 48 warps); the motion variants (object-ray
-// state) keep 4 and 64 registers; with the curve stage they take 3 and 80 (the
+// state) keep 4 and 64 registers (1280x720x16 motion frame 13.3 ms, 14.1 at 5); with the curve stage they take 3 and 80 (the
 // ribbon walk's state; 1280x720x8 hair frame 172.2 ms against 178.9 at 4
 // blocks and 64 registers).
 #define ANA_TRAVERSAL_BOUNDS \

@@ -80,20 +80,20 @@ __device__ __forceinline__ void box_slabs(const TriRay& r, const float (&lo)[3][
 }
 
 // Moller-Trumbore, BVHBackend::intersectTriangle.
-__device__ __forceinline__ bool tri_hit(const TriRay& r, float3 dir, float3 v0, float3 e1, float3 e2, float tmax,
+__device__ __forceinline__ bool tri_hit(float3 o, float3 dir, float tmin, float3 v0, float3 e1, float3 e2, float tmax,
                                         float& t, float& u, float& v) {
     float3 h = xcross(dir, e2);
     float a = xdot(e1, h);
     if (fabsf(a) < 1e-9f) return false;
     float f = xdiv(1.f, a);
-    float3 s = xsub3(r.o, v0);
+    float3 s = xsub3(o, v0);
     u = xmul(f, xdot(s, h));
     if (u < 0.f || u > 1.f) return false;
     float3 q = xcross(s, e1);
     v = xmul(f, xdot(dir, q));
     if (v < 0.f || xadd(u, v) > 1.f) return false;
     t = xmul(f, xdot(e2, q));
-    return t >= r.tmin && t <= tmax;
+    return t >= tmin && t <= tmax;
 }
 
 // Stack entry: interior node index, or a leaf (bit 31) with count-1 in bits
@@ -147,9 +147,9 @@ struct Counters {
 // the closest-hit count (shadow + MIS 107.0 ms at 8, 111.4 at 4, 108.1 at 12,
 // 111.9 at 16); the parked count serves the kernels that still park
 // (occlusion queries of ana_trace_batch on triangles). Kernels with
-// motion-blurred meshes, whose leaf tests invert interpolated matrices, keep
-// the phase until no lane descends (1280x720x16 motion frame: 25.9 ms against
-// 28.6 ms at 8 / 16 lanes). Hits and occlusion answers are unchanged.
+// motion-blurred meshes, whose leaf tests may invert interpolated matrices, keep
+// the phase until no lane descends (1280x720x16 motion frame: 13.3 ms against
+// 13.9 at 8 lanes). Hits and occlusion answers are unchanged.
 constexpr uint32_t kLeafPhaseLanes = 8;      // closest hit, any hit without parking
 constexpr uint32_t kLeafPhaseLanesAny = 16;  // any hit (parked leaves)
 
@@ -215,7 +215,8 @@ constexpr uint32_t kNoPrim = 0xFFFFFFFFu;
 //   stage on -4 .. -6 the ray frame's x and y axes
 //   -7, -8 (tangent, strand parameter) of the closest ribbon hit
 //   -9.x ray time, -9.y, -10 exact direction (motion)
-constexpr int kFrame = 10;
+//   -11.x motion mesh of the object ray in -11.y .. -14.x (origin, direction)
+constexpr int kFrame = 14;
 
 __device__ __forceinline__ uint2 pair(float a, float b) { return make_uint2(__float_as_uint(a), __float_as_uint(b)); }
 __device__ __forceinline__ float lo(uint2 p) { return __uint_as_float(p.x); }
@@ -252,6 +253,7 @@ __device__ __forceinline__ void trav_init(Traversal& T, const Ray& ray, uint32_t
     if (kMotion) {
         stack[-9] = pair(ray.time, ray.d.x);
         stack[-10] = pair(ray.d.y, ray.d.z);
+        stack[-11].x = kNoPrim;
     }
 }
 
@@ -370,20 +372,27 @@ __device__ __forceinline__ void enter_near_first(Traversal& T, float (&key)[4], 
 }
 
 // BVHBackend::makeObjectSpaceRay4: the world ray (origin, exact direction)
-// taken to the object space of motion mesh `mm` at the ray's time.
-__device__ __forceinline__ TriRay object_ray(const DevScene& S, uint32_t mm, const Traversal& T, const uint2* stack,
-                                             float tmax) {
+// taken to the object space of motion mesh `mm` at the ray's time. The origin
+// and the triangle tests' direction go to the lane's frame with the mesh: the
+// ray keeps them until it meets a leaf of another motion mesh (the reference
+// recomputes the same values per triangle). 1280x720x16 motion frame, with the
+// matrix interpolated and inverted at every leaf: extend 9.39 ms, shadow 6.04;
+// once per ray and run of leaves of a mesh: 5.48 and 3.55.
+__device__ __noinline__ void object_ray(const DevScene& S, uint32_t mm, float3 o, uint2* stack) {
     M4 o2w, w2o;
     const uint2 a = stack[-9], b = stack[-10];
     o2w_at(S, mm, lo(a), o2w);
     m4_inverse(o2w, w2o);
     Ray r;
-    r.o = m4_point(w2o, T.r.o);
+    r.o = m4_point(w2o, o);
     r.d = m4_vector(w2o, f3(hi(a), lo(b), hi(b)));
-    r.tmin = T.r.tmin;
-    r.tmax = tmax;
-    r.time = lo(a);
-    return make_tri_ray(r);
+    r.tmin = r.tmax = r.time = 0.f;
+    const TriRay q = make_tri_ray(r);
+    const float3 d = tri_dir(q);
+    stack[-11] = make_uint2(mm, __float_as_uint(q.o.x));
+    stack[-12] = pair(q.o.y, q.o.z);
+    stack[-13] = pair(d.x, d.y);
+    stack[-14] = pair(d.z, 0.f);
 }
 
 // Tests the triangles of leaf entry `leaf`; true when an any-hit query found
@@ -393,29 +402,26 @@ template <bool kAny, bool kCount, bool kMotion = false>
 __device__ __forceinline__ bool leaf_test(Traversal& T, const DevScene& S, uint32_t leaf, uint2* stack, Counters* cnt) {
     const float3 dir = frame_dir(stack);
     const uint32_t off = leaf & 0x01FFFFFFu, c = ((leaf >> 25) & 63u) + 1u;
-    // the object ray of the leaf's last motion mesh, reused while the mesh
-    // repeats (the same value the reference recomputes per triangle)
-    uint32_t cachedMM = 0xFFFFFFFFu;
-    TriRay ro;
-    float3 rodir;
+    uint32_t held = kNoPrim;  // motion mesh of (oo, od)
+    float3 oo, od;
     for (uint32_t i = off; i < off + c; ++i) {
         const float4* tp = S.tri_isect + 3 * size_t(i);
         float4 a = ldg4(tp), b = ldg4(tp + 1), e = ldg4(tp + 2);
         if (kCount) cnt->prims++;
         float t, u, v;
         const float tmax = kAny ? T.r.tmax : T.closest;
-        bool h;
-        if (kMotion && (__float_as_uint(a.w) & 0x80000000u)) {
+        const bool moving = kMotion && (__float_as_uint(a.w) & 0x80000000u);
+        if (moving) {
             const uint32_t mm = __float_as_uint(b.w);
-            if (mm != cachedMM) {
-                ro = object_ray(S, mm, T, stack, tmax);
-                rodir = tri_dir(ro);
-                cachedMM = mm;
+            if (mm != held) {
+                if (stack[-11].x != mm) object_ray(S, mm, T.r.o, stack);
+                const uint2 p = stack[-12], q = stack[-13];
+                oo = f3(hi(stack[-11]), lo(p), hi(p));
+                od = f3(lo(q), hi(q), lo(stack[-14]));
+                held = mm;
             }
-            h = tri_hit(ro, rodir, f3(a), f3(b), f3(e), tmax, t, u, v);
-        } else {
-            h = tri_hit(T.r, dir, f3(a), f3(b), f3(e), tmax, t, u, v);
         }
+        const bool h = tri_hit(moving ? oo : T.r.o, moving ? od : dir, T.r.tmin, f3(a), f3(b), f3(e), tmax, t, u, v);
         if (h) {
             T.closest = t;
             T.prim = i;
