@@ -1020,10 +1020,47 @@ __global__ void __launch_bounds__(256) k_adj_direct(const __grid_constant__ Para
     }
 }
 
+// Sums over the samples of a warp's 32 pixels, in sample order per pixel:
+// add(sample) gets each lane's pixel's samples of kWidth floats. The samples of
+// the pixels lie one pixel after the other; read by lane they are spp * kWidth
+// floats apart. Where the pixels are one run of a scene (`run`, from `base`) of
+// at least four tiles of samples, the warp reads kTileFloats of each pixel
+// together and hands them over in shared memory (32 rows of kTileFloats + 1):
+// film stage with camera rays of the 1920x1080x64 frame 3.46 -> 2.90 ms, of
+// 1280x720x16 with AOVs 0.68 -> 0.48. Fewer samples share sectors as they are,
+// and small films wait for the longer chain (256x256x16: 0.039 against 0.047 ms
+// at two tiles, 1280x720x8: 0.161 against 0.180 at one).
+constexpr uint32_t kTileFloats = 24;
+template <uint32_t kWidth, class Add>
+__device__ __forceinline__ void sum_samples(const float* base, bool run, uint32_t pixels, const float* mine,
+                                            uint32_t spp, float* tile, Add add) {
+    constexpr uint32_t kSamples = kTileFloats / kWidth;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (!run || spp < 4u * kSamples) {
+        for (uint32_t s = 0; s < spp; ++s) add(mine + kWidth * s);
+        return;
+    }
+    for (uint32_t s0 = 0; s0 < spp; s0 += kSamples) {
+        const uint32_t n = min(kSamples, spp - s0) * kWidth;  // floats per pixel in this tile
+        __syncwarp();
+        for (uint32_t j = lane; j < pixels * n; j += 32u) {
+            const uint32_t px = j / n, o = j - px * n;
+            tile[px * (kTileFloats + 1u) + o] = base[(size_t(px) * spp + s0) * kWidth + o];
+        }
+        __syncwarp();
+        if (lane < pixels)
+            for (uint32_t o = 0; o < n; o += kWidth) add(tile + lane * (kTileFloats + 1u) + o);
+    }
+}
+
 // Film accumulation (PathIntegrator.cpp:43-57 + Film::mergeTile, Film.cpp:34-56):
 // finite samples summed in sample order, weight = sample count.
 __global__ void __launch_bounds__(256) k_film(const __grid_constant__ Params p) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < p.chunk_pixels; q += gridDim.x * blockDim.x) {
+    __shared__ float tiles[8][32 * (kTileFloats + 1)];
+    float* const tile = tiles[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); q0 < p.chunk_pixels; q0 += gridDim.x * blockDim.x) {
+        const uint32_t pixels = min(32u, p.chunk_pixels - q0), q = q0 + min(lane, pixels - 1u);
         // the chunk's pixel run holding local pixel q
         uint32_t lo = 0, hi = p.num_segs;
         while (hi - lo > 1) {
@@ -1035,36 +1072,39 @@ __global__ void __launch_bounds__(256) k_film(const __grid_constant__ Params p) 
         const DevSceneRec& R = p.S.scenes[sg.scene];
         const uint32_t spp = R.spp;
         const uint32_t k = q - sg.local_pixel;
+        const bool run = __all_sync(0xFFFFFFFFu, lo == __shfl_sync(0xFFFFFFFFu, lo, 0));
+        const size_t mine = size_t(sg.local_path) + size_t(k) * spp, first = size_t(sg.local_path) + size_t(q0 - sg.local_pixel) * spp;
         float3 acc = f3(0.f, 0.f, 0.f);
         float lsq = 0.f;
-        const float* Lp = p.q.L + (size_t(sg.local_path) + size_t(k) * spp) * 3;
-        for (uint32_t s = 0; s < spp; ++s) {
-            float3 L = f3(Lp[3 * s], Lp[3 * s + 1], Lp[3 * s + 2]);
+        sum_samples<3>(p.q.L + first * 3, run, pixels, p.q.L + mine * 3, spp, tile, [&](const float* v) {
+            float3 L = f3(v[0], v[1], v[2]);
             if (is_finite3(L)) {
                 acc = acc + L;
                 float lum = luminance(L);
                 lsq += lum * lum;
             }
-        }
+        });
         const float invSPP = 1.f / float(spp);
         const size_t fi = film_index(R, sg.first_pixel + k);
         ana_film_pixel& f = p.film[fi];
         float w = float(spp);
-        f.r += (acc.x * invSPP) * w;
-        f.g += (acc.y * invSPP) * w;
-        f.b += (acc.z * invSPP) * w;
-        f.w += w;
-        f.sum_lum_sq += lsq;
+        if (lane < pixels) {
+            f.r += (acc.x * invSPP) * w;
+            f.g += (acc.y * invSPP) * w;
+            f.b += (acc.z * invSPP) * w;
+            f.w += w;
+            f.sum_lum_sq += lsq;
+        }
         if (p.aov) {
             // renderTile's AOV averages over every sample of the pass
             // (PathIntegrator.cpp:44-66), merged with weight 1 as
             // Film::mergeTile does (Film.cpp:58-70)
-            const float* A = p.q.aov + (size_t(sg.local_path) + size_t(k) * spp) * 6;
             float3 sa = f3(0.f, 0.f, 0.f), sn = f3(0.f, 0.f, 0.f);
-            for (uint32_t s = 0; s < spp; ++s) {
-                sa = xadd3(sa, f3(A[6 * s], A[6 * s + 1], A[6 * s + 2]));
-                sn = xadd3(sn, f3(A[6 * s + 3], A[6 * s + 4], A[6 * s + 5]));
-            }
+            sum_samples<6>(p.q.aov + first * 6, run, pixels, p.q.aov + mine * 6, spp, tile, [&](const float* v) {
+                sa = xadd3(sa, f3(v[0], v[1], v[2]));
+                sn = xadd3(sn, f3(v[3], v[4], v[5]));
+            });
+            if (lane >= pixels) continue;
             const float3 al = xmul3(sa, invSPP);
             float3 n = xmul3(sn, invSPP);
             const float len = __fsqrt_rn(xdot(n, n));
