@@ -330,6 +330,8 @@ struct ana_ctx {
     size_t adj_size = 0;
     uint32_t adj_cap = 0;
     float* adj_L = nullptr;
+    unsigned char* d_kept = nullptr;  // hits of the primal replay by bounce and path
+    size_t kept_size = 0;
     // pinned words of short copies (query records, counters), and the device
     // buffers of ray queries and resolved images
     unsigned char* pin = nullptr;
@@ -381,13 +383,14 @@ int ensure_buffer(ana_ctx* c, unsigned char** p, size_t* have, size_t need, cons
     drop_graph(c);
     void* mem = nullptr;
     cudaError_t e = cudaMalloc(&mem, need);
-    if (e == cudaErrorMemoryAllocation && (c->d_query || c->d_image)) {  // what is only kept makes room
+    if (e == cudaErrorMemoryAllocation && (c->d_query || c->d_image || c->d_kept)) {  // what is only kept makes room
         cudaGetLastError();
         CK(cudaStreamSynchronize(c->stream), "sync");
         cudaFree(c->d_query);
         cudaFree(c->d_image);
-        c->d_query = c->d_image = nullptr;
-        c->query_size = c->image_size = 0;
+        cudaFree(c->d_kept);
+        c->d_query = c->d_image = c->d_kept = nullptr;
+        c->query_size = c->image_size = c->kept_size = 0;
         e = cudaMalloc(&mem, need);
     }
     CK(e, what);
@@ -584,6 +587,32 @@ int ensure_adjoint(ana_ctx* c, uint32_t cap) {
     return ANA_OK;
 }
 
+// Room for the primal replay's hits of every bounce, which the adjoint replay
+// then does not trace again (512x512x16, depth 8: 604 MB; backward pass 10.7 -> 9.6
+// ms).
+// At most kKeepHits (a full chunk to depth 15), and only while the device has
+// the room: else the adjoint replay traces.
+constexpr size_t kKeepHits = size_t(8) << 30;
+bool ensure_kept(ana_ctx* c, uint32_t cap, uint32_t maxDepth) {
+    const size_t layer = align_up(size_t(cap) * 16), layers = size_t(maxDepth + 1) * (c->ds.has_curves ? 2 : 1);
+    if (layer * layers > kKeepHits) return false;
+    if (c->kept_size >= layer * layers && c->d_kept) return true;
+    if (c->d_kept) {
+        cudaStreamSynchronize(c->stream);
+        cudaFree(c->d_kept);
+        c->d_kept = nullptr;
+        c->kept_size = 0;
+    }
+    void* mem = nullptr;
+    if (cudaMalloc(&mem, layer * layers) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    c->d_kept = static_cast<unsigned char*>(mem);
+    c->kept_size = layer * layers;
+    return true;
+}
+
 // The batch render: descs[k] renders uploaded scene k into its film.
 // With adj_image (host, 3 floats per film pixel: dLoss / d pixel) it runs the
 // path-replay adjoint instead: per chunk a primal replay of the same paths
@@ -744,6 +773,9 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
     const size_t ncountAll = (backward ? 2 : 1) * ncount;
     rc = ensure_buffer(c, &c->d_counters, &c->counters_bytes, ncountAll * 4, "cudaMalloc(counters)");
     if (rc) return rc;
+    // after the buffers above, which may need its room; whether the adjoint
+    // replay takes the primal's hits
+    const bool keep = backward && ensure_kept(c, cap, maxDepth);
     uint32_t* counters = reinterpret_cast<uint32_t*>(c->d_counters);
     ana::Params p{};
     p.S = c->ds;
@@ -830,6 +862,11 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
         pa.a.d_image = reinterpret_cast<const float*>(c->d_adj_io);
         pa.a.grad = reinterpret_cast<float*>(c->d_adj_io + oGrad);
         pa.a.num_materials = uint32_t(c->h_mats.size());
+        if (keep) {
+            pa.a.kept = reinterpret_cast<float4*>(c->d_kept);
+            pa.a.kept_stride = align_up(size_t(cap) * 16) / 16;
+            pa.a.kept1 = pa.a.kept + pa.a.kept_stride * (maxDepth + 1);
+        }
         for (uint32_t k = 0; k < nchunks; ++k) {
             const ChunkPlan& cp = chunks[k];
             pa.chunk_first_path = cp.first_path;
@@ -843,8 +880,15 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
             pa.bounce = 0;
             timed(4, [&] { ana::launch_generate(pa, cfg, c->stream); });
             auto extend = [&](cudaStream_t s) { timed(0, [&] { ana::launch_extend(pa, cfg, s, false); }); };
+            auto extend_keep = [&](cudaStream_t s) {
+                extend(s);
+                if (keep) timed(4, [&] { ana::launch_keep_hits(pa, cfg, s); });
+            };
+            auto extend_adj = [&](cudaStream_t s) {
+                if (!keep) extend(s);
+            };
             bounces(
-                pa, extend, [&](cudaStream_t s) { timed(1, [&] { ana::launch_shade(pa, cfg, s); }); },
+                pa, extend_keep, [&](cudaStream_t s) { timed(1, [&] { ana::launch_shade(pa, cfg, s); }); },
                 [&](cudaStream_t s) {
                     timed(2, [&] { ana::launch_shadow(pa, cfg, s); });
                     timed(3, [&] { ana::launch_mis(pa, cfg, s); });
@@ -857,7 +901,7 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
             timed(4, [&] { ana::launch_generate(pa, cfg, c->stream); });
             timed(4, [&] { ana::launch_adj_init(pa, cfg, c->stream); });
             bounces(
-                pa, extend, [&](cudaStream_t s) { timed(1, [&] { ana::launch_shade_adj(pa, cfg, s); }); },
+                pa, extend_adj, [&](cudaStream_t s) { timed(1, [&] { ana::launch_shade_adj(pa, cfg, s); }); },
                 [&](cudaStream_t s) {
                     timed(2, [&] { ana::launch_shadow_adj(pa, cfg, s); });
                     timed(3, [&] { ana::launch_mis_adj(pa, cfg, s); });
@@ -1145,6 +1189,7 @@ void ana_destroy(ana_ctx* c) {
     cudaFree(c->d_err);
     cudaFree(c->d_adj);
     cudaFree(c->d_adj_io);
+    cudaFree(c->d_kept);
     cudaFree(c->d_query);
     cudaFree(c->d_image);
     if (c->pin) cudaFreeHost(c->pin);

@@ -507,7 +507,9 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
         float vPend[4] = {0.f, 0.f, 0.f, 0.f}, vEmit[3] = {0.f, 0.f, 0.f};
         if (i < n) {
             float4 qo = queue_load(p.q.ext_o[cur][i]), qd = queue_load(p.q.ext_d[cur][i]), qb = queue_load(p.q.ext_b[cur][i]);
-            float4 h0 = queue_load(p.q.hit0[i]);
+            float4 h0;
+            if (kAdj && p.a.kept) h0 = p.a.kept[b * p.a.kept_stride + (__float_as_uint(qo.w) - p.chunk_first_path)];
+            else h0 = queue_load(p.q.hit0[i]);
             const uint32_t pid = __float_as_uint(qo.w), meta = __float_as_uint(qd.w);
             const uint32_t sc = scene_bits(qb.w);
             const DevSceneRec& R = S.scenes[sc];
@@ -539,7 +541,9 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
             if (prim == kMiss) {
                 if (bounce == 0 || spec) Ladd = beta * scene_env(S, R, d);
             } else {
-                float4 h1 = (prim & 0x80000000u) ? p.q.hit1[i] : make_float4(0, 0, 0, 0);
+                float4 h1 = make_float4(0, 0, 0, 0);
+                if (prim & 0x80000000u)
+                    h1 = kAdj && p.a.kept ? p.a.kept1[b * p.a.kept_stride + (pid - p.chunk_first_path)] : p.q.hit1[i];
                 const float time = (kExtra && S.has_motion) ? path_time(R, pid) : 0.f;
                 SurfInt si = surf_int<kFiber, kExtra>(S, o, d, h0.x, prim, h0.z, h0.w, h1, time);
                 int mi = slot_material(S, R, si.slot);
@@ -965,6 +969,20 @@ __global__ void __launch_bounds__(256) k_adj_init(const __grid_constant__ Params
     }
 }
 
+// The adjoint replay walks the primal replay's paths: it takes their hits from
+// here instead of tracing them again (its queues are in another order, so the
+// hits are kept by path).
+__global__ void __launch_bounds__(256) k_keep_hits(const __grid_constant__ Params p) {
+    const uint32_t n = p.counters[p.bounce * kCountersPerBounce], cur = p.bounce & 1u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const size_t at = p.bounce * p.a.kept_stride + (__float_as_uint(p.q.ext_o[cur][i].w) - p.chunk_first_path);
+        const float4 h = p.q.hit0[i];
+        p.a.kept[at] = h;
+        const uint32_t prim = __float_as_uint(h.y);
+        if (prim != kMiss && (prim & 0x80000000u)) p.a.kept1[at] = p.q.hit1[i];
+    }
+}
+
 // Resolves the gradient payloads of one bounce once the shadow and MIS rays
 // are traced. NEE (unoccluded only): material albedo / roughness terms and
 // the area light's Le term. MIS: the material terms times the Li found, and
@@ -1256,6 +1274,7 @@ void prime_kernels() {
     prime(k_film);
     prime(k_adj_init);
     prime(k_adj_direct);
+    prime(k_keep_hits);
     prime(k_film_image);
     prime(k_aov_image);
     prime(k_extend<false, false, false>);
@@ -1428,6 +1447,9 @@ void launch_mis(const Params& p, const LaunchCfg& c, cudaStream_t s) {
 // the any-hit form the forward pass may use.
 void launch_adj_init(const Params& p, const LaunchCfg& c, cudaStream_t s) {
     k_adj_init<<<blocks_for(p.chunk_paths, 256, c.grid_cap), 256, 0, s>>>(p);
+}
+void launch_keep_hits(const Params& p, const LaunchCfg& c, cudaStream_t s) {
+    k_keep_hits<<<std::min(c.grid_cap, c.stage_grid), 256, 0, s>>>(p);
 }
 void launch_shade_adj(const Params& p, const LaunchCfg& c0, cudaStream_t s) {
     LaunchCfg c = c0;

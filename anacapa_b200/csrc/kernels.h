@@ -76,6 +76,11 @@ struct AdjQueues {
     const float* d_image;  // dLoss / d pixel, film layout (3 floats per pixel)
     float* grad;
     uint32_t num_materials;
+    // hits of the primal replay by bounce and path (kept + bounce * kept_stride +
+    // path of the chunk), null when they are not kept; kept1: curve hits' records
+    float4* kept;
+    float4* kept1;
+    size_t kept_stride;
 };
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
 
@@ -121,6 +126,8 @@ void launch_film(const Params& p, const LaunchCfg& c, cudaStream_t s);
 // with the gradient bookkeeping compiled in (identical sampling decisions),
 // the per-path delta set-up, and the resolution of the NEE and MIS gradient
 // payloads once their rays are traced.
+// Keeps a bounce's hits by path for the adjoint replay.
+void launch_keep_hits(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_adj_init(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_shade_adj(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_shadow_adj(const Params& p, const LaunchCfg& c, cudaStream_t s);
