@@ -427,10 +427,12 @@ void trim_scratch(unsigned char** p, size_t* have) {
 }
 
 // Wavefront buffers for `cap` paths.
+size_t queue_bytes(uint32_t cap) { return 14 * align_up(size_t(cap) * 16) + align_up(size_t(cap) * 12); }
+
 int ensure_queues(ana_ctx* c, uint32_t cap) {
     if (c->cap >= cap && c->d_queues) return ANA_OK;
     size_t f4 = size_t(cap) * 16;
-    size_t total = 14 * align_up(f4) + align_up(size_t(cap) * 12);
+    size_t total = queue_bytes(cap);
     size_t have = c->d_queues ? size_t(1) : 0;  // force reallocation
     if (c->d_queues) {
         CK(cudaStreamSynchronize(c->stream), "sync");
@@ -551,6 +553,26 @@ int upload_blob(ana_ctx* c, const Blob& B, const ana::DeviceTris* dt = nullptr) 
     return ANA_OK;
 }
 
+// Paths in flight per chunk unless the context names a number. The late bounces
+// of a chunk hold few rays, so more paths keep them filling the GPU: 2^25 (7.9
+// GB of queues), and twice that for a frame of more, while it takes at most an
+// eighth of the device's free memory. 1920x1080x64 frame: 263.0 ms at 2^25,
+// 255.3 at 2^26, 252.5 at 2^27, with its first pass in a new context 5 and 10 ms
+// sooner. The adjoint keeps 2^25: its own queues and kept hits come on top.
+constexpr uint32_t kChunkPaths = 1u << 25;
+uint32_t default_chunk(const ana_ctx* c, uint64_t totalPaths, bool backward) {
+    if (backward || totalPaths <= kChunkPaths) return kChunkPaths;
+    const uint32_t want = uint32_t(std::min<uint64_t>(totalPaths, 2 * uint64_t(kChunkPaths)));
+    if (c->d_queues && c->cap >= want) return want;
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return kChunkPaths;
+    }
+    if (c->d_queues) free += queue_bytes(c->cap);
+    return queue_bytes(want) <= free / 8 ? want : kChunkPaths;
+}
+
 struct ChunkPlan {
     uint32_t first_path, paths, pixels, seg_begin, seg_count;
 };
@@ -651,13 +673,14 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
     const bool count_work = (flags & ANA_RENDER_COUNT_WORK) != 0;
     const bool use_graph = (flags & ANA_RENDER_GRAPH) != 0 && !count_work;
     const bool timing = c->opts.timing != 0 && !use_graph;
-    // default chunk: 32M paths in flight (~8 GB of queues). Smaller chunks
-    // leave the late, sparse bounces of each chunk too few rays to fill the
-    // GPU (throughput scene: 772 ms/frame at 4M paths, 537 ms at 32M).
-    uint32_t cap = c->opts.chunk_paths ? c->opts.chunk_paths : (1u << 25);
+    uint32_t cap = c->opts.chunk_paths ? c->opts.chunk_paths : default_chunk(c, totalPaths, backward);
     cap = std::max(cap, maxSpp);
     if (uint64_t(cap) > totalPaths) cap = uint32_t(totalPaths);
     int rc = ensure_queues(c, cap);
+    if (rc == ANA_ERR_OOM && !c->opts.chunk_paths && cap > kChunkPaths) {
+        cap = std::max(kChunkPaths, maxSpp);
+        rc = ensure_queues(c, cap);
+    }
     if (rc) return rc;
     const size_t nparams = 8 * c->h_mats.size() + 4 * c->h_lights.size();
     const size_t oGrad = align_up(size_t(totalPixels) * 12);

@@ -272,7 +272,8 @@ typedef struct ana_ctx ana_ctx;
 
 typedef struct ana_device_opts {
     int device;              /* CUDA ordinal                                   */
-    uint32_t chunk_paths;    /* wavefront capacity in paths (0 = 2^25)         */
+    uint32_t chunk_paths;    /* wavefront capacity in paths (0 = 2^25, or 2^26 for
+                                larger frames on a device with room for it)    */
     uint32_t block_size;     /* threads per block of the shading kernel (0 = default 256;
                                 larger requests run 256-thread blocks)            */
     uint32_t timing;         /* 1: record per-stage CUDA-event times           */
