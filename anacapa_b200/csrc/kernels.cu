@@ -463,37 +463,60 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
     // alone, with the environment added while listing, gained the throughput
     // frame another 0.3 ms and cost closed scenes 3 %.
     constexpr bool kFilter = !kAdj;
-    __shared__ uint32_t s_list[kFilter ? 2 * kShadeBlock : 1];
-    __shared__ uint32_t s_listed;
-    const bool filter = kFilter && b > 0;
-    uint32_t base = blockIdx.x * blockDim.x, listed = 0;
+    // kSort: two lists, standard_surface hits and the others, so that a warp
+    // shades one kind (but for the one warp where the lists meet) and appends
+    // rays that leave one kind of surface. Batches of glass, alpha masks or
+    // motion mix the kinds (1279x719x16 glass frame 9.39 -> 9.24 ms, 1280x720x16
+    // motion frame 12.41 -> 12.16, where shading loses 0.2 and shadow rays gain 0.3); the classes the
+    // other kernels are compiled for mostly do not.
+    constexpr bool kSort = kFilter && kExtra && !kFiber;
+    constexpr uint32_t kList = 2 * kShadeBlock;
+    __shared__ uint32_t s_list[kFilter ? kList : 1];
+    __shared__ uint32_t s_listed[2];
+    const bool filter = kFilter && (b > 0 || kSort);
+    uint32_t base = blockIdx.x * blockDim.x, listed[2] = {0, 0};
     if (filter) {
-        if (threadIdx.x == 0) s_listed = 0;
+        if (threadIdx.x < 2) s_listed[threadIdx.x] = 0;
         __syncthreads();
     }
     while (true) {
         uint32_t i = n;
         if (filter) {
-            while (listed < blockDim.x && base < n) {
+            while (listed[0] + listed[1] < blockDim.x && base < n) {
                 const uint32_t e = base + threadIdx.x;
                 bool live = false;
+                uint32_t kind = 0;
                 if (e < n) {
-                    live = __float_as_uint(p.q.hit0[e].y) != kMiss;
+                    const uint32_t prim = __float_as_uint(p.q.hit0[e].y);
+                    live = b == 0 || prim != kMiss;
                     if (!live) live = (__float_as_uint(p.q.ext_d[cur][e].w) >> 8) & 1u;  // specular: sees the environment
+                    if (kSort && prim != kMiss && !(prim & 0x80000000u)) {
+                        const DevSceneRec& R = S.scenes[scene_bits(p.q.ext_b[cur][e].w)];
+                        const int mi = slot_material(S, R, hit_slot(S, prim));
+                        kind = mi >= 0 && S.materials[mi].type == ANA_MAT_STANDARD ? 1u : 0u;
+                    }
                 }
-                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, live), lane = threadIdx.x & 31u;
-                uint32_t at = 0;
-                if (lane == 0 && mask) at = atomicAdd(&s_listed, __popc(mask));
-                at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(mask & ((1u << lane) - 1u));
-                if (live) s_list[at] = e;
+                const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+#pragma unroll
+                for (uint32_t q = 0; q < (kSort ? 2u : 1u); ++q) {
+                    const bool mine = live && kind == q;
+                    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, mine);
+                    uint32_t at = 0;
+                    if (lane == 0 && mask) at = atomicAdd(&s_listed[q], __popc(mask));
+                    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(mask & lt);
+                    if (mine) s_list[q ? kList - 1u - at : at] = e;
+                    listed[q] += __syncthreads_count(mine);
+                }
                 base += stride;
-                listed += __syncthreads_count(live);
             }
-            const uint32_t take = min(listed, blockDim.x);
-            if (take == 0) break;
-            listed -= take;
-            if (threadIdx.x < take) i = s_list[listed + threadIdx.x];
-            if (threadIdx.x == 0) s_listed = listed;
+            // the second list grows down from the end: threads take from it first
+            const uint32_t take1 = kSort ? min(listed[1], blockDim.x) : 0u, take0 = min(listed[0], blockDim.x - take1);
+            if (take0 + take1 == 0) break;
+            listed[0] -= take0;
+            listed[1] -= take1;
+            if (threadIdx.x < take1) i = s_list[kList - 1u - (listed[1] + threadIdx.x)];
+            else if (threadIdx.x < take0 + take1) i = s_list[listed[0] + threadIdx.x - take1];
+            if (threadIdx.x < 2) s_listed[threadIdx.x] = listed[threadIdx.x];
         } else {
             if (base >= n) break;
             i = base + threadIdx.x;
@@ -1362,13 +1385,14 @@ void launch_extend(const Params& p, const LaunchCfg& c, cudaStream_t s, bool cou
         else ps ? ext_launch<false, false, true>(p, c, s) : ext_launch<false, false, false>(p, c, s);
     }
 }
-// Past bounce 0 the blocks list the entries to shade before shading them
-// (k_shade), which needs several tiles per block: one resident wave instead of
-// the four that balance blocks of one tile (two waves measured the same on the
-// throughput frame and cost the glass frame's shade stage 2.5 %).
+// Past bounce 0, and in the sorting kernel (`sorts`) always, the blocks list the
+// entries to shade before shading them (k_shade), which needs several tiles per
+// block: one resident wave instead of the four that balance blocks of one tile
+// (two waves measured the same on the throughput frame and cost the glass
+// frame's shade stage 2.5 %).
 template <class K>
-static void shade_launch(K k, const Params& p, const LaunchCfg& c, int grid, cudaStream_t s) {
-    if (p.bounce > 0) grid = std::min(grid, resident_grid(k) * (kPersistBlock / c.block));
+static void shade_launch(K k, const Params& p, const LaunchCfg& c, int grid, cudaStream_t s, bool sorts = false) {
+    if (p.bounce > 0 || sorts) grid = std::min(grid, resident_grid(k) * (kPersistBlock / c.block));
     k<<<grid, c.block, 0, s>>>(p);
 }
 void launch_shade(const Params& p, const LaunchCfg& c0, cudaStream_t s) {
@@ -1386,7 +1410,7 @@ void launch_shade(const Params& p, const LaunchCfg& c0, cudaStream_t s) {
         else if ((f & ~kLambArea) == 0) shade_launch(k_shade<false, true, false, kLambArea>, p, c, g, s);
         else shade_launch(k_shade<false, true, false>, p, c, g, s);
     } else {
-        if (extra) shade_launch(k_shade<false, false, true>, p, c, g, s);
+        if (extra) shade_launch(k_shade<false, false, true>, p, c, g, s, true);
         else if ((f & ~kStdDome) == 0) shade_launch(k_shade<false, false, false, kStdDome>, p, c, g, s);
         else if ((f & ~kLambArea) == 0) shade_launch(k_shade<false, false, false, kLambArea>, p, c, g, s);
         else shade_launch(k_shade<false, false, false>, p, c, g, s);
