@@ -34,7 +34,7 @@ def build(reference=None, quiet=True):
     whether the libraries are already built."""
     libs = [os.path.join(REF_DIR, n) for n in ("libanacapa_ref.so", "libanacapa_ref_nocontract.so")]
     reference = reference or os.environ.get("ANACAPA_REFERENCE")
-    if not reference or not os.path.isdir(reference):
+    if not reference or not os.path.isdir(os.path.join(reference, "src")):  # absent, or an empty mount
         return all(os.path.exists(p) for p in libs)
     subprocess.run(["make", "-C", HERE, "ref", f"REF={reference}"], check=True,
                    stdout=subprocess.DEVNULL if quiet else None)
