@@ -370,6 +370,19 @@ void drop_graph(ana_ctx* c) {
     c->graph.key.clear();
 }
 
+// Frees what is only kept between calls (query and image buffers, the last
+// adjoint's hits): other allocations come first.
+bool free_kept(ana_ctx* c) {
+    if (!c->d_query && !c->d_image && !c->d_kept) return false;
+    cudaStreamSynchronize(c->stream);
+    cudaFree(c->d_query);
+    cudaFree(c->d_image);
+    cudaFree(c->d_kept);
+    c->d_query = c->d_image = c->d_kept = nullptr;
+    c->query_size = c->image_size = c->kept_size = 0;
+    return true;
+}
+
 // Grows a device buffer (contents are not kept). Any cached graph refers to
 // the old address, so it is dropped.
 int ensure_buffer(ana_ctx* c, unsigned char** p, size_t* have, size_t need, const char* what) {
@@ -383,15 +396,9 @@ int ensure_buffer(ana_ctx* c, unsigned char** p, size_t* have, size_t need, cons
     drop_graph(c);
     void* mem = nullptr;
     cudaError_t e = cudaMalloc(&mem, need);
-    if (e == cudaErrorMemoryAllocation && (c->d_query || c->d_image || c->d_kept)) {  // what is only kept makes room
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        CK(cudaStreamSynchronize(c->stream), "sync");
-        cudaFree(c->d_query);
-        cudaFree(c->d_image);
-        cudaFree(c->d_kept);
-        c->d_query = c->d_image = c->d_kept = nullptr;
-        c->query_size = c->image_size = c->kept_size = 0;
-        e = cudaMalloc(&mem, need);
+        if (free_kept(c)) e = cudaMalloc(&mem, need);
     }
     CK(e, what);
     *p = static_cast<unsigned char*>(mem);
@@ -414,7 +421,12 @@ int ensure_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need, con
     *p = nullptr;
     *have = 0;
     void* mem = nullptr;
-    CK(cudaMalloc(&mem, need), what);
+    cudaError_t e = cudaMalloc(&mem, need);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (free_kept(c)) e = cudaMalloc(&mem, need);
+    }
+    CK(e, what);
     *p = static_cast<unsigned char*>(mem);
     *have = need;
     return ANA_OK;
@@ -1305,6 +1317,7 @@ int ana_upload_scene_device(ana_ctx* c, const ana_scene_desc* d) {
     try {
         rc = ana::prepare_scene(*d, pp->P, err, true);
         if (rc == ANA_OK && pp->P.tris_on_device) {
+            free_kept(c);  // the build's memory comes first, and the kept hits are the old scene's
             const uint32_t maxLeaf = d->max_leaf_tris ? d->max_leaf_tris : 4;
             rc = ana::build_tris_on_device(*d, maxLeaf, c->stream, dt, err);
             pp->P.dev_tri_nodes = dt.num_nodes;

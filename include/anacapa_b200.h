@@ -388,10 +388,11 @@ int ana_trace_batch_timed(ana_ctx* ctx, const float* rays, const float* times, s
                           int occlusion_only, int rays_on_device);
 
 /* ana_trace_batch without any device allocation (no counterpart in the
- * reference). ana_trace_batch takes a temporary device buffer per call
- * (cudaMalloc / cudaFree); this variant stages the rays, the hits and its
- * counters in a fixed scratch array that lives in the library's module
- * memory, one per device. It is for callers that cannot allocate device
+ * reference). ana_trace_batch grows a device buffer of its context when a
+ * query is larger than those before it (and frees one of more than 256 MiB
+ * when the call ends), and long copies take pinned host memory; this variant
+ * stages the rays, the hits and its counters in a fixed scratch array that
+ * lives in the library's module memory, one per device. It is for callers that cannot allocate device
  * memory at the moment they trace: a viewer answering a pick or hover query
  * while a frame renders on another stream (cudaFree waits for all work on
  * the device, so the query would stall until the frame ends), and a process
