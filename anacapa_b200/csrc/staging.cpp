@@ -25,7 +25,13 @@ public:
 
 private:
     static constexpr int kThreads = 4;
-    static constexpr size_t kChunk = size_t(1) << 20;
+    // Page-locking a set is part of the first large copy of a program's only
+    // context: 8 MiB takes 4-8 ms, 1 MiB 1-2.6. With chunks of 1 MiB (8 MiB a
+    // set) a new context's first query of 200,000 rays took 10.1 ms and its next
+    // ones 3.2, of 2^20 rays 15 and 3.1-4.5; with 256 KiB 7.2 and 3.3, 8.8 and
+    // 4.3; with 128 KiB 4.4 and 3.4, 6.7 and 5.3; through the driver's own path
+    // 6.1 and 5.7, 6-12 and 5.5-12.
+    static constexpr size_t kChunk = size_t(1) << 17;
     cudaError_t run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, bool out);
     int device_;
     unsigned char* pinned_ = nullptr;

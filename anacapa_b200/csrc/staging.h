@@ -10,10 +10,9 @@ namespace ana {
 // caller's memory, whose pages are often touched there for the first time. The
 // driver's own path for pageable memory does both in turn on one thread.
 //
-// Sets of chunks (8 MiB pinned), streams and events are shared by the contexts
-// of a process: a copy takes an idle set of its device, or makes one (several
-// milliseconds, which a context's first film would pay otherwise), and gives it
-// back. Two idle sets at most are kept, and none once the last context is gone.
+// Sets of chunks (1 MiB pinned), streams and events are shared by the contexts
+// of a process: a copy takes an idle set of its device, or makes one (1-3
+// milliseconds), and gives it back. Two idle sets at most are kept, and none once the last context is gone.
 
 // Every context holds one reference (stage_retain at its creation).
 void stage_retain();
