@@ -913,6 +913,9 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
             pa.q.L = c->q.L;
             pa.counters = counters + size_t(k) * rows * ana::kCountersPerBounce;
             pa.bounce = 0;
+            if (keep)  // no path has walked yet
+                cudaMemset2DAsync(pa.a.kept, pa.a.kept_stride * 16, ana::kUnwalkedByte, size_t(cp.paths) * 16,
+                                  size_t(maxDepth) + 1, c->stream);
             timed(4, [&] { ana::launch_generate(pa, cfg, c->stream); });
             auto extend = [&](cudaStream_t s) { timed(0, [&] { ana::launch_extend(pa, cfg, s, false); }); };
             auto extend_keep = [&](cudaStream_t s) {

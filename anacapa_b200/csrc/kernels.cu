@@ -561,7 +561,12 @@ __global__ void __launch_bounds__(kShadeBlock, (!kAdj && !kFiber) ? (kFeat == kF
                     vPend[3] = sum3(wr);
                 }
             }
-            if (prim == kMiss) {
+            if (kAdj && prim == kUnwalked) {
+                // The primal replay's path ended before this bounce: all of L
+                // is gathered, and there is no hit to read. The two replays run
+                // differently compiled kernels; a roulette decision within
+                // their rounding may differ.
+            } else if (prim == kMiss) {
                 if (bounce == 0 || spec) Ladd = beta * scene_env(S, R, d);
             } else {
                 float4 h1 = make_float4(0, 0, 0, 0);

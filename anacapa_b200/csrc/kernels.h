@@ -77,12 +77,15 @@ struct AdjQueues {
     float* grad;
     uint32_t num_materials;
     // hits of the primal replay by bounce and path (kept + bounce * kept_stride +
-    // path of the chunk), null when they are not kept; kept1: curve hits' records
+    // path of the chunk), null when they are not kept; kept1: curve hits' records.
+    // kUnwalked in the place of prim: the primal replay's path ended before
     float4* kept;
     float4* kept1;
     size_t kept_stride;
 };
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+constexpr int kUnwalkedByte = 0xFE;
+constexpr uint32_t kUnwalked = 0xFEFEFEFEu;  // neither a miss nor an index (both below 2^25)
 
 struct Params {
     DevScene S;
