@@ -20,7 +20,7 @@ def _build():
         out = os.path.join(_dir.name, "libfake.so")
         src = [os.path.join(build.CSRC, f) for f in ("capi.cpp", "prepare.cpp", "staging.cpp", "film_io.cpp")]
         subprocess.run([os.environ.get("CXX", "g++"), "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread",
-                        "-ffp-contract=off", f"-I{build.CUDA_HOME}/include", f"-I{build.ROOT}/include",
+                        "-ffp-contract=off", "-Wl,-Bsymbolic", f"-I{build.CUDA_HOME}/include", f"-I{build.ROOT}/include",
                         f"-I{build.CSRC}", *src, os.path.join(HERE, "fake_device.cpp"), "-o", out, "-lz"], check=True)
     return os.path.join(_dir.name, "libfake.so")
 
