@@ -370,16 +370,25 @@ void drop_graph(ana_ctx* c) {
     c->graph.key.clear();
 }
 
+// Frees the adjoint's kept hits.
+void free_hits(ana_ctx* c) {
+    if (!c->d_kept) return;
+    cudaStreamSynchronize(c->stream);
+    cudaFree(c->d_kept);
+    c->d_kept = nullptr;
+    c->kept_size = 0;
+}
+
 // Frees what is only kept between calls (query and image buffers, the last
 // adjoint's hits): other allocations come first.
 bool free_kept(ana_ctx* c) {
     if (!c->d_query && !c->d_image && !c->d_kept) return false;
+    free_hits(c);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->d_query);
     cudaFree(c->d_image);
-    cudaFree(c->d_kept);
-    c->d_query = c->d_image = c->d_kept = nullptr;
-    c->query_size = c->image_size = c->kept_size = 0;
+    c->d_query = c->d_image = nullptr;
+    c->query_size = c->image_size = 0;
     return true;
 }
 
@@ -483,6 +492,7 @@ int ensure_queues(ana_ctx* c, uint32_t cap) {
 // from a device build (device-to-device) and the blob holds the rest.
 int upload_blob(ana_ctx* c, const Blob& B, const ana::DeviceTris* dt = nullptr) {
     CK(cudaSetDevice(c->device), "cudaSetDevice");
+    free_hits(c);  // the old scene's
     int rc = ensure_buffer(c, &c->d_scene, &c->d_scene_size, B.size, "cudaMalloc(scene)");
     if (rc) return rc;
     if (dt) {
@@ -622,28 +632,31 @@ int ensure_adjoint(ana_ctx* c, uint32_t cap) {
 }
 
 // Room for the primal replay's hits of every bounce, which the adjoint replay
-// then does not trace again (512x512x16, depth 8: 604 MB; backward pass 10.7 -> 9.6
-// ms).
-// At most kKeepHits (a full chunk to depth 15), and only while the device has
-// the room: else the adjoint replay traces.
-constexpr size_t kKeepHits = size_t(8) << 30;
+// then does not trace again (512x512x16, depth 8: 604 MB; backward pass 10.7 -> 9.7
+// ms). The room is held between passes: 2.4 GB of 1024x1024x16 allocated and
+// freed by each pass took the 3.3 ms that they save (36.5 ms a pass; 33.3 held,
+// 36.6 traced). At most kKeepHits, and a sixteenth of the device's free memory,
+// which the caller's other allocators share: else the adjoint replay traces. A
+// pass that needs less than half of it gives the rest back.
+constexpr size_t kKeepHits = size_t(4) << 30;
 bool ensure_kept(ana_ctx* c, uint32_t cap, uint32_t maxDepth) {
     const size_t layer = align_up(size_t(cap) * 16), layers = size_t(maxDepth + 1) * (c->ds.has_curves ? 2 : 1);
-    if (layer * layers > kKeepHits) return false;
-    if (c->kept_size >= layer * layers && c->d_kept) return true;
-    if (c->d_kept) {
-        cudaStreamSynchronize(c->stream);
-        cudaFree(c->d_kept);
-        c->d_kept = nullptr;
-        c->kept_size = 0;
+    const size_t need = layer * layers;
+    if (c->kept_size >= need && c->kept_size / 2 <= need && c->d_kept) return true;
+    free_hits(c);
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
+    if (need > kKeepHits || need > free / 16) return false;
     void* mem = nullptr;
-    if (cudaMalloc(&mem, layer * layers) != cudaSuccess) {
+    if (cudaMalloc(&mem, need) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     c->d_kept = static_cast<unsigned char*>(mem);
-    c->kept_size = layer * layers;
+    c->kept_size = need;
     return true;
 }
 

@@ -495,7 +495,11 @@ int ana_render_adaptive(ana_ctx* ctx, const ana_render_desc* frame, uint32_t til
  * radiance L and once to propagate the adjoint (Vicini, Speierer, Jakob 2021:
  * sampling decisions, pdfs, MIS weights and roulette are held fixed), and
  * reduces the per-path gradients per warp in FP32 before atomic adds. Hair
- * parameters and the dome are not differentiated. */
+ * parameters and the dome are not differentiated. The first replay's hits are
+ * kept for the second where they take at most 4 GiB and a sixteenth of the
+ * device's free memory (16 bytes, with curves 32, per path of a chunk and
+ * bounce); that room is held for the next backward pass, until a scene is
+ * uploaded, a pass of less than half of it, or the context's end. */
 typedef struct ana_diff_params {
     float* albedo;
     float* roughness;

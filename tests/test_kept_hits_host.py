@@ -26,3 +26,74 @@ def test_paths_the_primal_did_not_walk_have_no_hit(chunk, curves):
             r.backward(np.ones((h, w, 3), np.float32))
         assert L.fake_good_records() == 2 * w * h * spp * (depth + 1)
         assert L.fake_bad_records() == 0
+
+
+W, H, SPP, DEPTH = 40, 30, 4, 5
+ROOM = -(-W * H * SPP * 16 // 256) * 256 * (DEPTH + 1)
+
+
+def _backward(r, w=W, h=H):
+    r.forward(w, h, SPP, DEPTH)
+    r.backward(np.ones((h, w, 3), np.float32))
+
+
+def _held_without_hits(sc):
+    with fake_device() as L, closing(api.Renderer()) as r:
+        L.fake_fail(b"cudaMemGetInfo", 0, -1)
+        r.upload(sc)
+        _backward(r)
+        assert L.fake_good_records() == 0
+        return L.fake_held()
+
+
+def test_hits_are_kept_in_a_part_of_free_memory():
+    """Room for them is taken only where it is a sixteenth of what is free, and
+    the pass does without it where it is not, or cannot be had."""
+    sc = S.differentiable(W, H, SPP, DEPTH, subdiv=1)
+    other = _held_without_hits(sc)
+    for free, kept in ((16 * ROOM, True), (16 * ROOM - 16, False)):
+        with fake_device(capacity=other + free) as L, closing(api.Renderer()) as r:
+            r.upload(sc)
+            _backward(r)
+            assert (L.fake_good_records() > 0) == kept
+            assert L.fake_held() == other + (ROOM if kept else 0)
+    with fake_device() as L, closing(api.Renderer()) as r:
+        r.upload(sc)
+        r.forward(W, H, SPP, DEPTH)
+        # queues, image, counters of the pass come first; the last one is the room
+        L.fake_fail(b"cudaMalloc", 3, 1)
+        r.backward(np.ones((H, W, 3), np.float32))
+        assert L.fake_good_records() == 0 and L.fake_held() == other
+
+
+def test_room_for_hits_is_given_back():
+    sc = S.differentiable(W, H, SPP, DEPTH, subdiv=1)
+    other = _held_without_hits(sc)
+    with fake_device() as L, closing(api.Renderer()) as r:
+        r.upload(sc)
+        for _ in range(3):
+            _backward(r)
+            assert L.fake_held() == other + ROOM
+        allocations = L.fake_calls(b"cudaMalloc")
+        _backward(r)
+        assert L.fake_calls(b"cudaMalloc") == allocations
+        _backward(r, 20, 10)  # a smaller frame: less than half of it
+        assert L.fake_held() - other < ROOM // 4
+        _backward(r)
+        r.upload(sc)
+        assert L.fake_held() == other
+        _backward(r)
+        r.trace(np.ones((4, 8), np.float32))  # its own buffer
+        assert L.fake_held() > other + ROOM
+
+
+def test_other_allocations_come_before_the_room_for_hits():
+    sc = S.differentiable(W, H, SPP, DEPTH, subdiv=1)
+    with fake_device() as L, closing(api.Renderer()) as r:
+        r.upload(sc)
+        _backward(r)
+        held = L.fake_held()
+        L.fake_fail(b"cudaMalloc", 0, 1)
+        out = r.trace(np.full((5000, 8), 3.0, np.float32))
+        assert (out["t"] == 3).all()
+        assert L.fake_held() < held
