@@ -1069,7 +1069,8 @@ int render_items(ana_ctx* c, const std::vector<Item>& items, uint64_t totalPixel
     for (uint32_t k = 0; k < nchunks * (backward ? 2u : 1u); ++k)
         for (uint32_t b = 0; b < rows; ++b) {
             const uint32_t* cc = c->h_counters.data() + (size_t(k) * rows + b) * ana::kCountersPerBounce;
-            if (b <= maxDepth) st.extend_rays += cc[0];
+            // kept hits: the adjoint replay (the second half) traces none
+            if (b <= maxDepth && !(keep && k >= nchunks)) st.extend_rays += cc[0];
             st.shadow_rays += cc[1];
             st.mis_rays += cc[2];
             if (cc[0]) st.bounces = std::max(st.bounces, b + 1);

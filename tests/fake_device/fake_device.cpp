@@ -280,7 +280,8 @@ void launch_extend(const Params& p, const LaunchCfg&, cudaStream_t, bool) {
     g_extend_rays += p.counters[p.bounce * kCountersPerBounce];
 }
 void launch_shade(const Params& p, const LaunchCfg&, cudaStream_t) {
-    p.counters[(p.bounce + 1) * kCountersPerBounce] = entries(p.chunk_paths, p.bounce + 1);
+    if (p.bounce < p.S.scenes[0].max_depth)
+        p.counters[(p.bounce + 1) * kCountersPerBounce] = entries(p.chunk_paths, p.bounce + 1);
 }
 void launch_shadow(const Params&, const LaunchCfg&, cudaStream_t) {}
 void launch_mis(const Params&, const LaunchCfg&, cudaStream_t) {}

@@ -30,3 +30,31 @@ def test_room_with_other_scenes_hits(gpu):
     finally:
         used.close()
         fresh.close()
+
+
+def test_statistics_tell_kept_from_traced_hits(gpu):
+    """The two routes of the adjoint replay, told apart by the rays they trace,
+    give the same gradient. 2^14 paths to depth 24 fit the room for hits; the
+    same frame to depth 255 in one chunk of 2^21 paths does not."""
+    d = np.random.default_rng(6).normal(size=(128, 128, 3)).astype(np.float32) / (128 * 128)
+    for (w, h, spp), depth, kept in (((128, 128, 1), 24, True), ((512, 512, 8), 255, False)):
+        sc = S.differentiable(w, h, spp, depth, subdiv=2)
+        out = []
+        for chunk in (1 << 21, 1 << 12 if kept else 1 << 16):
+            r = api.Renderer(chunk_paths=chunk)
+            try:
+                r.upload(sc)
+                r.forward(w, h, spp, depth)
+                forward = r.stats().extend_rays
+                g = r.backward(np.resize(d, (h, w, 3)))
+                traced = r.stats().extend_rays / forward
+                if kept or chunk < 1 << 21:
+                    assert traced == 1
+                else:
+                    assert 1.99 < traced < 2.01
+                out.append(g)
+            finally:
+                r.close()
+        for k in out[0]:
+            a, b = out[0][k].astype(np.float64), out[1][k].astype(np.float64)
+            assert np.linalg.norm(a - b) <= 1e-3 * np.linalg.norm(b) + 1e-12, k

@@ -97,3 +97,18 @@ def test_other_allocations_come_before_the_room_for_hits():
         out = r.trace(np.full((5000, 8), 3.0, np.float32))
         assert (out["t"] == 3).all()
         assert L.fake_held() < held
+
+
+@pytest.mark.parametrize("kept", [True, False])
+def test_statistics_count_the_rays_that_are_traced(kept):
+    sc = S.differentiable(W, H, SPP, DEPTH, subdiv=1)
+    with fake_device() as L, closing(api.Renderer(chunk_paths=1000)) as r:
+        if not kept:
+            L.fake_fail(b"cudaMemGetInfo", 0, -1)
+        r.upload(sc)
+        r.forward(W, H, SPP, DEPTH)
+        forward = L.fake_extend_rays()
+        assert r.stats().extend_rays == forward > 0
+        r.backward(np.ones((H, W, 3), np.float32))
+        assert r.stats().extend_rays == L.fake_extend_rays() - forward == (1 if kept else 2) * forward
+        assert r.stats().bounces == DEPTH + 1
