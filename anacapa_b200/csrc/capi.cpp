@@ -1721,6 +1721,7 @@ static int trace_batch(ana_ctx* c, const float* rays, const float* times, size_t
     if (rc) return rc;
     uint32_t herr = 0;
     const cudaError_t e = run_query(c, c->d_query, rays, times, n, out, occlusion, on_device, true, herr);
+    if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // copies of the caller's page-locked memory
     trim_scratch(&c->d_query, &c->query_size);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace batch");
     if (herr) return fail(c, ANA_ERR_DEVICE_CHECK, "ana_trace_batch: traversal stack overflow on the device");
@@ -1756,7 +1757,10 @@ int ana_trace_batch_noalloc(ana_ctx* c, const float* rays, size_t n, ana_hit* ou
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_trace_batch_noalloc: scratch address (cudaGetSymbolAddress)");
     uint32_t herr = 0;
     e = run_query(c, base, rays, nullptr, n, out, occlusion, 0, false, herr);
-    if (e != cudaSuccess) return cuda_fail(c, e, "ana_trace_batch_noalloc");
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(c->stream);
+        return cuda_fail(c, e, "ana_trace_batch_noalloc");
+    }
     if (herr) return fail(c, ANA_ERR_DEVICE_CHECK, "ana_trace_batch_noalloc: traversal stack overflow on the device");
     return ANA_OK;
 }
@@ -1783,6 +1787,7 @@ int ana_bsdf_batch(ana_ctx* c, const ana_material* material, const ana_bsdf_quer
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = ana::stage_read(out, dr, n * sizeof(ana_bsdf_result), c->stream, c->device);
+    if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // copies of the caller's page-locked memory
     trim_scratch(&c->d_query, &c->query_size);
     if (e != cudaSuccess) return cuda_fail(c, e, "ana_bsdf_batch");
     return ANA_OK;

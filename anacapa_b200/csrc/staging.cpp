@@ -160,8 +160,26 @@ void give_back(std::unique_ptr<HostStage> s) {
     // else freed here
 }
 
+// Whether every copy of the range goes through the driver's own buffers:
+// neither page-locked nor managed nor device memory, which it moves directly
+// (1920x1080 film into page-locked memory 0.74 ms, through the chunks 3.0; 2^20
+// page-locked rays and hits 2.6 and 4.9).
+bool pageable(const void* p, size_t bytes) {
+    const unsigned char* const ends[2] = {static_cast<const unsigned char*>(p),
+                                          static_cast<const unsigned char*>(p) + bytes - 1};
+    for (const unsigned char* q : ends) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+            cudaGetLastError();
+            return true;
+        }
+        if (a.type == cudaMemoryTypeUnregistered) return true;
+    }
+    return false;
+}
+
 cudaError_t staged(void* dst, const void* src, size_t bytes, cudaStream_t st, int device, bool out) {
-    if (bytes >= kStageMin) {
+    if (bytes >= kStageMin && pageable(out ? dst : src, bytes)) {
         if (std::unique_ptr<HostStage> s = take(device)) {
             const cudaError_t e = s->copy(dst, src, bytes, st, out);
             if (e == cudaSuccess) give_back(std::move(s));  // after an error its events say nothing: freed

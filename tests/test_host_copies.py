@@ -1,0 +1,76 @@
+"""Copies between host memory and the device: which route a buffer takes."""
+from contextlib import closing
+
+import numpy as np
+import pytest
+
+from anacapa_b200 import api
+from anacapa_b200 import scenes as S
+from tests.fake_device import DEVICE, HOST, MANAGED, fake_device
+
+W, H = 320, 240  # films of 1.5 MB
+
+
+def _rendered(r):
+    sc = S.cornell(W, H, 1, 2)
+    r.upload(sc)
+    r.render(W, H, 1, 2)
+
+
+def _film(L, r, kind):
+    out = np.empty((H, W, 5), np.float32)
+    if kind is not None:
+        L.fake_mark(out.ctypes.data, out.nbytes, kind)
+    before, chunks = L.fake_direct_bytes(), L.fake_calls(b"cudaEventSynchronize")
+    api.check(L.ana_film_read(r.h, out.ctypes.data, W * H), r.h)
+    L.fake_mark(out.ctypes.data, 0, -1)
+    assert np.array_equal(out[..., 0].ravel(), np.arange(W * H, dtype=np.float32))
+    return L.fake_direct_bytes() - before, L.fake_calls(b"cudaEventSynchronize") - chunks
+
+
+@pytest.mark.parametrize("kind", [HOST, MANAGED, DEVICE])
+def test_memory_that_the_driver_moves_directly_is_left_to_it(kind):
+    with fake_device() as L, closing(api.Renderer()) as r:
+        _rendered(r)
+        assert _film(L, r, kind) == (W * H * 20, 0)
+        assert _film(L, r, None)[0] == 0  # pageable: through the pinned chunks
+
+
+def test_page_locked_queries():
+    n = 70_000
+    rays, out = np.random.default_rng(0).random((n, 8), np.float32), np.zeros(n, api.HIT_DTYPE)
+    with fake_device() as L, closing(api.Renderer()) as r:
+        _rendered(r)
+        before = L.fake_direct_bytes()
+        api.check(L.ana_trace_batch(r.h, rays.ctypes.data, n, out.ctypes.data, 0, 0), r.h)
+        pageable = L.fake_direct_bytes() - before
+        for a in (rays, out):
+            L.fake_mark(a.ctypes.data, a.nbytes, HOST)
+        want, out[:] = out.copy(), np.zeros((), api.HIT_DTYPE)
+        api.check(L.ana_trace_batch(r.h, rays.ctypes.data, n, out.ctypes.data, 0, 0), r.h)
+        assert L.fake_direct_bytes() - before - 2 * pageable == 2 * 32 * n
+        assert np.array_equal(out, want) and np.array_equal(out["t"], rays[:, 0])
+        # of the rays only the first half is page-locked: none is assumed to be
+        L.fake_mark(rays.ctypes.data, rays.nbytes // 2, HOST)
+        before = L.fake_direct_bytes()
+        api.check(L.ana_trace_batch(r.h, rays.ctypes.data, n, out.ctypes.data, 0, 0), r.h)
+        assert L.fake_direct_bytes() - before - pageable == 32 * n  # the hits
+        for a in (rays, out):
+            L.fake_mark(a.ctypes.data, 0, -1)
+
+
+def test_a_failed_query_leaves_no_copy_of_the_callers_memory_running():
+    n = 70_000
+    rays, out = np.ones((n, 8), np.float32), np.zeros(n, api.HIT_DTYPE)
+    with fake_device() as L, closing(api.Renderer()) as r:
+        _rendered(r)
+        for a in (rays, out):
+            L.fake_mark(a.ctypes.data, a.nbytes, HOST)
+        waits = L.fake_calls(b"cudaStreamSynchronize")
+        L.fake_fail(b"cudaMemcpyAsync", 2, 1)  # after the scene record and the rays: the hits
+        assert L.ana_trace_batch(r.h, rays.ctypes.data, n, out.ctypes.data, 0, 0) == api.ANA_ERR_CUDA
+        assert L.fake_calls(b"cudaStreamSynchronize") == waits + 1
+        api.check(L.ana_trace_batch(r.h, rays.ctypes.data, n, out.ctypes.data, 0, 0), r.h)
+        assert (out["t"] == 1).all()
+        for a in (rays, out):
+            L.fake_mark(a.ctypes.data, 0, -1)
