@@ -424,8 +424,8 @@ constexpr size_t kKeepBytes = size_t(256) << 20;
 
 // Grows a buffer that no captured graph refers to (contents are not kept).
 // Its last call is complete: these calls wait for the stream.
-int ensure_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need, const char* what) {
-    if (*have >= need && *p) return ANA_OK;
+cudaError_t grow_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need) {
+    if (*have >= need && *p) return cudaSuccess;
     if (*p) cudaFree(*p);
     *p = nullptr;
     *have = 0;
@@ -435,9 +435,13 @@ int ensure_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need, con
         cudaGetLastError();
         if (free_kept(c)) e = cudaMalloc(&mem, need);
     }
-    CK(e, what);
+    if (e != cudaSuccess) return e;
     *p = static_cast<unsigned char*>(mem);
     *have = need;
+    return cudaSuccess;
+}
+int ensure_scratch(ana_ctx* c, unsigned char** p, size_t* have, size_t need, const char* what) {
+    CK(grow_scratch(c, p, have, need), what);
     return ANA_OK;
 }
 void trim_scratch(unsigned char** p, size_t* have) {
@@ -445,6 +449,29 @@ void trim_scratch(unsigned char** p, size_t* have) {
     cudaFree(*p);
     *p = nullptr;
     *have = 0;
+}
+
+// Device buffer of a resolved image (ana_ctx::d_image); false: none to be had.
+bool image_buffer(ana_ctx* c, size_t pixels) {
+    if (grow_scratch(c, &c->d_image, &c->image_size, pixels * 12) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// Where the device has no room for a resolved image, its pixels are resolved
+// here: each(pixel, floats) for all `count` records of `width` floats.
+template <class Each>
+int read_pixels(ana_ctx* c, const float* dev, size_t width, size_t count, const char* what, Each each) {
+    const size_t slice = std::min<size_t>(count, size_t(1) << 14);
+    std::unique_ptr<float[]> h(new (std::nothrow) float[slice * width]);
+    if (!h) return fail(c, ANA_ERR_OOM, std::string(what) + ": host allocation failed");
+    for (size_t i0 = 0; i0 < count; i0 += slice) {
+        const size_t n = std::min(slice, count - i0);
+        CK(cudaMemcpyAsync(h.get(), dev + i0 * width, n * width * 4, cudaMemcpyDeviceToHost, c->stream), what);
+        CK(cudaStreamSynchronize(c->stream), what);
+        for (size_t i = 0; i < n; ++i) each(i0 + i, h.get() + i * width);
+    }
+    return ANA_OK;
 }
 
 // Wavefront buffers for `cap` paths.
@@ -1570,13 +1597,21 @@ int ana_aov_read(ana_ctx* c, float* albedo, float* normal, size_t count) {
     if (count != c->film_pixels)
         return fail(c, ANA_ERR_INVALID_ARG, "ana_aov_read: count != pixels of the last render");
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    int rc = ensure_scratch(c, &c->d_image, &c->image_size, count * 12, "cudaMalloc(resolved image)");
-    if (rc) return rc;
+    const float* const film = reinterpret_cast<const float*>(c->aov_film);
+    if (!image_buffer(c, count))  // PixelAccumulator::resolve
+        return read_pixels(c, film, 8, count, "AOV D2H", [&](size_t i, const float* px) {
+            for (int l = 0; l < 2; ++l) {
+                float* out = l ? normal : albedo;
+                if (!out) continue;
+                const float w = px[4 * l + 3], inv = w > 0.f ? 1.f / w : 0.f;
+                for (int k = 0; k < 3; ++k) out[3 * i + k] = w > 0.f ? px[4 * l + k] * inv : 0.f;
+            }
+        });
     float* const img = reinterpret_cast<float*>(c->d_image);
-    for (int l = 0; l < 2; ++l) {  // PixelAccumulator::resolve, 12 of 16 bytes per pixel and layer
+    for (int l = 0; l < 2; ++l) {  // the same on the device, 12 of 16 bytes per pixel and layer
         float* out = l ? normal : albedo;
         if (!out) continue;
-        ana::launch_aov_image(reinterpret_cast<const float*>(c->aov_film), uint32_t(count), l, img, c->stream);
+        ana::launch_aov_image(film, uint32_t(count), l, img, c->stream);
         CK(cudaGetLastError(), "AOV resolve");
         CK(ana::stage_read(out, img, count * 12, c->stream, c->device), "AOV D2H");
     }
@@ -1856,8 +1891,10 @@ int ana_forward(ana_ctx* c, const ana_render_desc* d, const ana_diff_params* par
     c->fwd_valid = true;
     if (image) {
         const size_t n = size_t(d->width) * d->height;
-        rc = ensure_scratch(c, &c->d_image, &c->image_size, n * 12, "cudaMalloc(resolved image)");
-        if (rc) return rc;
+        if (!image_buffer(c, n))  // Film::getPixel
+            return read_pixels(c, reinterpret_cast<const float*>(c->film), 5, n, "image D2H", [&](size_t i, const float* px) {
+                for (int k = 0; k < 3; ++k) image[3 * i + k] = px[3] > 0.f ? px[k] / px[3] : 0.f;
+            });
         ana::launch_film_image(c->film_px(), uint32_t(n), reinterpret_cast<float*>(c->d_image), c->stream);
         CK(cudaGetLastError(), "film resolve");
         CK(ana::stage_read(image, c->d_image, n * 12, c->stream, c->device), "image D2H");

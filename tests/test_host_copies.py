@@ -74,3 +74,27 @@ def test_a_failed_query_leaves_no_copy_of_the_callers_memory_running():
         assert (out["t"] == 1).all()
         for a in (rays, out):
             L.fake_mark(a.ctypes.data, 0, -1)
+
+
+@pytest.mark.parametrize("size", [(W, H), (129, 127), (1, 1)])
+def test_images_resolve_without_device_memory(size):
+    """A device without room for a resolved image: the same pixels."""
+    w, h = size
+    sc = S.differentiable(w, h, 1, 2, subdiv=1)
+    images = []
+    with fake_device() as L:
+        for full in (False, True):
+            with closing(api.Renderer()) as r:
+                r.upload(sc)
+                r.render(w, h, 1, 2, aovs=True)
+                held = L.fake_held()
+                if full:
+                    L.fake_fail(b"cudaMalloc", 0, -1)
+                images.append([*r.aovs(w, h), r.forward(w, h, 1, 2)])
+                assert (L.fake_held() == held) == full
+    for a, b in zip(*images):
+        assert np.array_equal(a, b)
+    al, nr, img = images[1]
+    i = np.arange(w * h, dtype=np.float32)
+    assert np.array_equal(al[..., 0].ravel(), i / 4) and (nr == 0).all()
+    assert np.array_equal(img[..., 2].ravel(), 3 * i / 2)
