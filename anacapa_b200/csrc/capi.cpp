@@ -1248,7 +1248,7 @@ int ana_create(ana_ctx** out, const ana_device_opts* opts) {
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
     ana::prime_kernels();
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(e, "kernel load");
-    ana::stage_retain();
+    ana::stage_retain(c->device);
     *out = c;
     return ANA_OK;
 }
@@ -1272,7 +1272,7 @@ void ana_destroy(ana_ctx* c) {
     cudaFree(c->d_query);
     cudaFree(c->d_image);
     if (c->pin) cudaFreeHost(c->pin);
-    ana::stage_release();
+    ana::stage_release(c->device);
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);

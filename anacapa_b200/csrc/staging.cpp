@@ -7,7 +7,6 @@
 #include <new>
 #include <system_error>
 #include <thread>
-#include <vector>
 
 namespace ana {
 
@@ -125,39 +124,46 @@ cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream
     return e;
 }
 
-// The sets not in use. Never destroyed itself: at the process's end the driver
-// may be gone before it.
+// The sets not in use, by device: a copy of another device's context finds its
+// own idle. Never destroyed itself (at the process's end the driver may be gone
+// before it), and nothing in it allocates.
+constexpr int kDevices = 64;  // sets of higher ordinals are made for each copy
+constexpr int kIdle = 2;
 struct Pool {
     std::mutex mu;
-    int contexts = 0;
-    std::vector<std::unique_ptr<HostStage>> idle;
+    struct {
+        int contexts = 0;
+        std::unique_ptr<HostStage> idle[kIdle];
+    } dev[kDevices];
 };
 Pool& pool() {
-    static Pool* p = new Pool;
+    alignas(Pool) static unsigned char mem[sizeof(Pool)];
+    static Pool* p = new (mem) Pool;
     return *p;
 }
-constexpr size_t kIdle = 2;
 
 std::unique_ptr<HostStage> take(int device) {
-    {
+    if (device < kDevices) {
         std::lock_guard<std::mutex> lk(pool().mu);
-        auto& idle = pool().idle;
-        for (size_t i = 0; i < idle.size(); ++i)
-            if (idle[i]->device() == device) {
-                std::unique_ptr<HostStage> s = std::move(idle[i]);
-                idle.erase(idle.begin() + std::ptrdiff_t(i));
-                return s;
-            }
+        for (std::unique_ptr<HostStage>& s : pool().dev[device].idle)
+            if (s) return std::move(s);
     }
     std::unique_ptr<HostStage> s(new (std::nothrow) HostStage(device));
     if (s && !s->make()) s.reset();
     return s;
 }
 
-void give_back(std::unique_ptr<HostStage> s) {
+// Keeps the set, or leaves it to the caller to free.
+void give_back(std::unique_ptr<HostStage>& s) {
+    if (s->device() >= kDevices) return;
     std::lock_guard<std::mutex> lk(pool().mu);
-    if (pool().contexts > 0 && pool().idle.size() < kIdle) pool().idle.push_back(std::move(s));
-    // else freed here
+    auto& d = pool().dev[s->device()];
+    if (d.contexts == 0) return;
+    for (std::unique_ptr<HostStage>& slot : d.idle)
+        if (!slot) {
+            slot = std::move(s);
+            return;
+        }
 }
 
 // Whether every copy of the range goes through the driver's own buffers:
@@ -182,7 +188,7 @@ cudaError_t staged(void* dst, const void* src, size_t bytes, cudaStream_t st, in
     if (bytes >= kStageMin && pageable(out ? dst : src, bytes)) {
         if (std::unique_ptr<HostStage> s = take(device)) {
             const cudaError_t e = s->copy(dst, src, bytes, st, out);
-            if (e == cudaSuccess) give_back(std::move(s));  // after an error its events say nothing: freed
+            if (e == cudaSuccess) give_back(s);  // after an error its events say nothing: freed
             return e;
         }
     }
@@ -193,14 +199,18 @@ cudaError_t staged(void* dst, const void* src, size_t bytes, cudaStream_t st, in
 
 }  // namespace
 
-void stage_retain() {
+void stage_retain(int device) {
+    if (device >= kDevices) return;
     std::lock_guard<std::mutex> lk(pool().mu);
-    pool().contexts++;
+    pool().dev[device].contexts++;
 }
-void stage_release() {
-    std::vector<std::unique_ptr<HostStage>> gone;
+void stage_release(int device) {
+    if (device >= kDevices) return;
+    std::unique_ptr<HostStage> gone[kIdle];  // freed after the lock
     std::lock_guard<std::mutex> lk(pool().mu);
-    if (--pool().contexts == 0) gone.swap(pool().idle);
+    auto& d = pool().dev[device];
+    if (--d.contexts == 0)
+        for (int i = 0; i < kIdle; ++i) gone[i] = std::move(d.idle[i]);
 }
 
 cudaError_t stage_read(void* dst, const void* src, size_t bytes, cudaStream_t st, int device) {

@@ -15,11 +15,12 @@ namespace ana {
 //
 // Sets of chunks (1 MiB pinned), streams and events are shared by the contexts
 // of a process: a copy takes an idle set of its device, or makes one (1-3
-// milliseconds), and gives it back. Two idle sets at most are kept, and none once the last context is gone.
+// milliseconds), and gives it back. Two idle sets at most are kept per device,
+// and none once the device's last context is gone.
 
 // Every context holds one reference (stage_retain at its creation).
-void stage_retain();
-void stage_release();
+void stage_retain(int device);
+void stage_release(int device);
 
 // dst (host) <- src (device), after the work queued on st. Complete on return.
 cudaError_t stage_read(void* dst, const void* src, size_t bytes, cudaStream_t st, int device);

@@ -1,5 +1,5 @@
 """Copies between host memory and the device: which route a buffer takes."""
-from contextlib import closing
+from contextlib import ExitStack, closing
 
 import numpy as np
 import pytest
@@ -98,3 +98,28 @@ def test_images_resolve_without_device_memory(size):
     i = np.arange(w * h, dtype=np.float32)
     assert np.array_equal(al[..., 0].ravel(), i / 4) and (nr == 0).all()
     assert np.array_equal(img[..., 2].ravel(), 3 * i / 2)
+
+
+def test_idle_sets_are_kept_by_device():
+    """Contexts on four devices, whose copies alternate: no set is made twice,
+    a device's sets go with its last context, and page-locked memory with them."""
+    with fake_device() as L, ExitStack() as stack:
+        rs = [stack.enter_context(closing(api.Renderer(device=d))) for d in (0, 1, 2, 3, 3)]
+        for r in rs:
+            _rendered(r)
+            r.film(W, H)
+        made = L.fake_calls(b"cudaHostAlloc")
+        for _ in range(3):
+            for r in rs:
+                r.film(W, H)
+        assert L.fake_calls(b"cudaHostAlloc") == made
+        freed = L.fake_calls(b"cudaStreamDestroy")
+        rs.pop().close()  # the fourth device has another context
+        assert L.fake_calls(b"cudaStreamDestroy") == freed + 2  # its own two
+        rs.pop().close()
+        assert L.fake_calls(b"cudaStreamDestroy") > freed + 4
+        again = stack.enter_context(closing(api.Renderer(device=3)))
+        _rendered(again)
+        made = L.fake_calls(b"cudaHostAlloc")
+        again.film(W, H)
+        assert L.fake_calls(b"cudaHostAlloc") == made + 1
