@@ -5,7 +5,6 @@
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 
 namespace ana {
@@ -114,7 +113,7 @@ cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream
     int started = 1;
     try {
         for (; started < threads; ++started) pool[started] = std::thread(work, started);
-    } catch (const std::system_error&) {  // no more threads to be had: this one does their part
+    } catch (...) {  // no thread or no memory for one to be had: this one does their part
     }
     work(0);
     for (int t = started; t < threads; ++t) work(t);

@@ -41,6 +41,7 @@ def fake_device(capacity=1 << 30):
         L.fake_fail.argtypes = [C.c_char_p, C.c_long, C.c_long]
         L.fake_calls.argtypes = [C.c_char_p]
         L.fake_mark.argtypes = [C.c_void_p, C.c_size_t, C.c_int]
+        L.fake_fail_new.argtypes = [C.c_long]
         L.fake_reset(capacity)
         yield L
         assert L.fake_held() == 0, "device memory of closed contexts"

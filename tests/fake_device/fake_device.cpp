@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 
 #include "build.h"
@@ -36,8 +37,14 @@ cudaError_t ret(cudaError_t e) {
     if (e != cudaSuccess) t_last = e;
     return e;
 }
+thread_local bool t_own = false;  // in the fake's own bookkeeping
+
 // Counts the call; true when it is to fail.
 bool called(const char* fn) {
+    struct Own {
+        Own() { t_own = true; }
+        ~Own() { t_own = false; }
+    } own;
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     g_calls[fn]++;
     auto it = g_faults.find(fn);
@@ -72,7 +79,17 @@ T* handle() {
     return reinterpret_cast<T*>(next.fetch_add(1));
 }
 
+std::atomic<long> g_new{-1};  // allocations to let pass before one fails, -1: none fails
+
 }  // namespace
+
+void* operator new(size_t n) {
+    if (!t_own && g_new >= 0 && g_new-- == 0) throw std::bad_alloc();
+    if (void* p = std::malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 extern "C" {
 
@@ -105,6 +122,7 @@ long fake_direct_bytes() { return g_direct_bytes; }
 long fake_extend_rays() { return g_extend_rays; }
 long fake_bad_records() { return g_bad_records; }
 long fake_good_records() { return g_good_records; }
+void fake_fail_new(long after) { g_new = after; }
 void fake_other_capture(int on) { g_other_captures = on != 0; }
 long fake_capture_broken() { return g_capture_broken; }
 

@@ -123,3 +123,16 @@ def test_idle_sets_are_kept_by_device():
         made = L.fake_calls(b"cudaHostAlloc")
         again.film(W, H)
         assert L.fake_calls(b"cudaHostAlloc") == made + 1
+
+
+@pytest.mark.parametrize("threads", [0, 1, 2])
+def test_a_copy_without_memory_for_its_threads(threads):
+    """The calling thread copies the part of those that could not be started."""
+    with fake_device() as L, closing(api.Renderer()) as r:
+        _rendered(r)
+        want = r.film(W, H)
+        out = np.zeros_like(want)
+        L.fake_fail_new(threads)
+        rc = L.ana_film_read(r.h, out.ctypes.data, W * H)
+        L.fake_fail_new(-1)
+        assert rc == api.ANA_OK and np.array_equal(out, want)
