@@ -34,8 +34,7 @@ def fake_device(capacity=1 << 30):
         L = api.lib()
         for name in ("fake_held", "fake_largest"):
             getattr(L, name).restype = C.c_size_t
-        for name in ("fake_calls", "fake_direct_bytes", "fake_extend_rays", "fake_bad_records", "fake_good_records",
-                     "fake_capture_broken"):
+        for name in ("fake_calls", "fake_direct_bytes", "fake_extend_rays", "fake_bad_records", "fake_good_records"):
             getattr(L, name).restype = C.c_long
         L.fake_reset.argtypes = [C.c_size_t]
         L.fake_fail.argtypes = [C.c_char_p, C.c_long, C.c_long]

@@ -28,9 +28,6 @@ std::map<std::string, long> g_calls;
 std::map<std::string, std::pair<long, long>> g_faults;  // calls to let pass, calls to fail
 size_t g_capacity = size_t(1) << 30, g_held = 0, g_largest = 0;
 long g_direct_bytes = 0, g_extend_rays = 0, g_bad_records = 0, g_good_records = 0;
-bool g_other_captures = false;
-long g_capture_broken = 0;
-thread_local cudaStreamCaptureMode t_mode = cudaStreamCaptureModeGlobal;
 thread_local cudaError_t t_last = cudaSuccess;
 
 cudaError_t ret(cudaError_t e) {
@@ -55,14 +52,6 @@ bool called(const char* fn) {
     }
     if (it->second.second == 0) return false;
     it->second.second--;
-    return true;
-}
-// A call that another thread's capture in global mode forbids, unless this
-// thread has chosen the relaxed mode.
-bool forbidden() {
-    if (!g_other_captures || t_mode == cudaStreamCaptureModeRelaxed) return false;
-    std::lock_guard<std::recursive_mutex> lk(g_mu);
-    g_capture_broken++;
     return true;
 }
 const Range* range_of(const void* p, uintptr_t* base = nullptr) {
@@ -100,8 +89,7 @@ void fake_reset(size_t capacity) {
     g_faults.clear();
     g_capacity = capacity;
     g_largest = 0;
-    g_direct_bytes = g_extend_rays = g_bad_records = g_good_records = g_capture_broken = 0;
-    g_other_captures = false;
+    g_direct_bytes = g_extend_rays = g_bad_records = g_good_records = 0;
 }
 void fake_fail(const char* fn, long after, long times) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
@@ -123,13 +111,10 @@ long fake_extend_rays() { return g_extend_rays; }
 long fake_bad_records() { return g_bad_records; }
 long fake_good_records() { return g_good_records; }
 void fake_fail_new(long after) { g_new = after; }
-void fake_other_capture(int on) { g_other_captures = on != 0; }
-long fake_capture_broken() { return g_capture_broken; }
 
 // ---- the runtime ----------------------------------------------------------
 cudaError_t cudaMalloc(void** p, size_t n) {
     if (called("cudaMalloc")) return ret(cudaErrorMemoryAllocation);
-    if (forbidden()) return ret(cudaErrorStreamCaptureUnsupported);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (n > g_capacity || g_held > g_capacity - n) return ret(cudaErrorMemoryAllocation);
     *p = std::aligned_alloc(256, (n + 255) & ~size_t(255));
@@ -142,7 +127,6 @@ cudaError_t cudaMalloc(void** p, size_t n) {
 cudaError_t cudaFree(void* p) {
     called("cudaFree");
     if (!p) return cudaSuccess;
-    if (forbidden()) return ret(cudaErrorStreamCaptureUnsupported);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     auto it = g_ranges.find(reinterpret_cast<uintptr_t>(p));
     if (it == g_ranges.end()) return ret(cudaErrorInvalidValue);
@@ -153,7 +137,6 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) {
     if (called("cudaHostAlloc")) return ret(cudaErrorMemoryAllocation);
-    if (forbidden()) return ret(cudaErrorStreamCaptureUnsupported);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     *p = std::aligned_alloc(4096, (n + 4095) & ~size_t(4095));
     g_ranges[reinterpret_cast<uintptr_t>(*p)] = {n, cudaMemoryTypeHost};
@@ -161,7 +144,6 @@ cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) {
 }
 cudaError_t cudaFreeHost(void* p) {
     called("cudaFreeHost");
-    if (forbidden()) return ret(cudaErrorStreamCaptureUnsupported);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     g_ranges.erase(reinterpret_cast<uintptr_t>(p));
     std::free(p);
@@ -251,10 +233,6 @@ cudaError_t cudaGetLastError() {
     const cudaError_t e = t_last;
     t_last = cudaSuccess;
     return e;
-}
-cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
-    std::swap(*m, t_mode);
-    return cudaSuccess;
 }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
