@@ -24,15 +24,21 @@ public:
 private:
     static constexpr int kThreads = 4;
     // Page-locking a set is part of the first large copy of a program's only
-    // context: 8 MiB takes 4-8 ms, 1 MiB 1-2.6. With chunks of 1 MiB (8 MiB a
-    // set) a new context's first query of 200,000 rays took 10.1 ms and its next
-    // ones 3.2, of 2^20 rays 15 and 3.1-4.5; with 256 KiB 7.2 and 3.3, 8.8 and
-    // 4.3; with 128 KiB 4.4 and 3.4, 6.7 and 5.3; through the driver's own path
-    // 6.1 and 5.7, 6-12 and 5.5-12.
-    static constexpr size_t kChunk = size_t(1) << 17;
+    // context: 8 MiB takes 4-10 ms, 1 MiB 1-2.6. Copies through 128 KiB chunks
+    // (1 MiB a set) are slower: a 1920x1080 film into used pages takes 3.06 ms,
+    // through 1 MiB chunks 1.6, through the driver's own path 2.35; 960x540 0.87,
+    // 0.45, 0.60; 2^20 rays and hits 4.9, 2.4, 4.6. That is 8 MiB's cost for
+    // every 128-256 MiB copied, so a set that has copied kGrowAfter takes the
+    // larger chunks: no program pays much more than twice the better choice.
+    static constexpr size_t kSmallChunk = size_t(1) << 17, kLargeChunk = size_t(1) << 20;
+    static constexpr size_t kGrowAfter = size_t(128) << 20;
+    void grow();
     cudaError_t run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, bool out);
     int device_;
-    unsigned char* pinned_ = nullptr;
+    unsigned char* pinned_ = nullptr;  // the chunks in use
+    unsigned char* small_ = nullptr;   // the first ones: freeing them may wait for the device
+    unsigned char* large_ = nullptr;
+    size_t chunk_ = kSmallChunk, copied_ = 0;
     cudaStream_t stream_[kThreads] = {};
     cudaEvent_t done_[kThreads][2] = {};
     cudaEvent_t begin_ = nullptr;
@@ -49,13 +55,14 @@ HostStage::~HostStage() {
             if (e) cudaEventDestroy(e);
     }
     if (begin_) cudaEventDestroy(begin_);
-    if (pinned_) cudaFreeHost(pinned_);
+    if (small_) cudaFreeHost(small_);
+    if (large_) cudaFreeHost(large_);
 }
 
 bool HostStage::make() {
     void* p = nullptr;
-    bool ok = cudaHostAlloc(&p, kThreads * 2 * kChunk, cudaHostAllocPortable) == cudaSuccess;
-    if (ok) pinned_ = static_cast<unsigned char*>(p);
+    bool ok = cudaHostAlloc(&p, kThreads * 2 * kSmallChunk, cudaHostAllocPortable) == cudaSuccess;
+    if (ok) pinned_ = small_ = static_cast<unsigned char*>(p);
     ok = ok && cudaEventCreateWithFlags(&begin_, cudaEventDisableTiming) == cudaSuccess;
     for (int t = 0; ok && t < kThreads; ++t) {
         ok = cudaStreamCreateWithFlags(&stream_[t], cudaStreamNonBlocking) == cudaSuccess;
@@ -65,15 +72,27 @@ bool HostStage::make() {
     return ok;
 }
 
+// Without memory for it, asked again after as much has been copied.
+void HostStage::grow() {
+    copied_ = 0;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kThreads * 2 * kLargeChunk, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    pinned_ = large_ = static_cast<unsigned char*>(p);
+    chunk_ = kLargeChunk;
+}
+
 // Thread t's chunks t, t + threads, ...
 cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigned char* src, size_t bytes, bool out) {
     cudaError_t e = cudaSetDevice(device_);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_[t], begin_, 0);
-    const size_t chunks = (bytes + kChunk - 1) / kChunk, step = size_t(threads);
-    unsigned char* slot[2] = {pinned_ + size_t(2 * t) * kChunk, pinned_ + size_t(2 * t + 1) * kChunk};
-    auto size_of = [&](size_t k) { return std::min(kChunk, bytes - k * kChunk); };
+    const size_t chunks = (bytes + chunk_ - 1) / chunk_, step = size_t(threads);
+    unsigned char* slot[2] = {pinned_ + size_t(2 * t) * chunk_, pinned_ + size_t(2 * t + 1) * chunk_};
+    auto size_of = [&](size_t k) { return std::min(chunk_, bytes - k * chunk_); };
     auto fetch = [&](size_t k, int s) {
-        cudaError_t r = cudaMemcpyAsync(slot[s], src + k * kChunk, size_of(k), cudaMemcpyDeviceToHost, stream_[t]);
+        cudaError_t r = cudaMemcpyAsync(slot[s], src + k * chunk_, size_of(k), cudaMemcpyDeviceToHost, stream_[t]);
         return r == cudaSuccess ? cudaEventRecord(done_[t][s], stream_[t]) : r;
     };
     int s = 0;
@@ -82,14 +101,14 @@ cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigne
         for (size_t k = size_t(t); e == cudaSuccess && k < chunks; k += step, s ^= 1) {
             if (k + step < chunks) e = fetch(k + step, s ^ 1);
             if (e == cudaSuccess) e = cudaEventSynchronize(done_[t][s]);
-            if (e == cudaSuccess) std::memcpy(dst + k * kChunk, slot[s], size_of(k));
+            if (e == cudaSuccess) std::memcpy(dst + k * chunk_, slot[s], size_of(k));
         }
     } else {
         for (size_t k = size_t(t), i = 0; e == cudaSuccess && k < chunks; k += step, ++i, s ^= 1) {
             if (i >= 2) e = cudaEventSynchronize(done_[t][s]);  // the slot's last copy has left it
             if (e != cudaSuccess) break;
-            std::memcpy(slot[s], src + k * kChunk, size_of(k));
-            e = cudaMemcpyAsync(dst + k * kChunk, slot[s], size_of(k), cudaMemcpyHostToDevice, stream_[t]);
+            std::memcpy(slot[s], src + k * chunk_, size_of(k));
+            e = cudaMemcpyAsync(dst + k * chunk_, slot[s], size_of(k), cudaMemcpyHostToDevice, stream_[t]);
             if (e == cudaSuccess) e = cudaEventRecord(done_[t][s], stream_[t]);
         }
     }
@@ -97,14 +116,16 @@ cudaError_t HostStage::run(int t, int threads, unsigned char* dst, const unsigne
     return e == cudaSuccess ? f : e;
 }
 
-// 1920x1080 film (41 MB) into fresh pages 4.9 -> 2.4 ms (1.8 into used ones, 23
-// GB/s), 960x540 film (10 MB) into used pages 0.38; 2^20 rays in and hits out (32
-// MB each) with their traversal 7.5 -> 4.6 ms.
+// Into fresh pages the driver's own path takes 8.9 ms for a 1920x1080 film (41 MB)
+// and 9.7 for 2^20 rays and hits (32 MB each) with their traversal; small chunks
+// 4.0 and 5.9, large ones 2.7-3.4 and 3.8-4.2.
 cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream_t st, bool out) {
+    if (!large_ && copied_ >= kGrowAfter) grow();
+    copied_ += bytes;
     cudaError_t e = cudaEventRecord(begin_, st);
     if (e != cudaSuccess) return e;
     const unsigned cores = std::thread::hardware_concurrency();
-    const int threads = int(std::min<size_t>({size_t(kThreads), std::max<size_t>(1, cores / 2), (bytes + kChunk - 1) / kChunk}));
+    const int threads = int(std::min<size_t>({size_t(kThreads), std::max<size_t>(1, cores / 2), (bytes + chunk_ - 1) / chunk_}));
     cudaError_t result[kThreads] = {};
     auto work = [&](int t) {
         result[t] = run(t, threads, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, out);

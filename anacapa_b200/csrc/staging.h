@@ -13,9 +13,9 @@ namespace ana {
 // thread. Memory that it moves directly (page-locked, managed) and short copies
 // are left to it.
 //
-// Sets of chunks (1 MiB pinned), streams and events are shared by the contexts
-// of a process: a copy takes an idle set of its device, or makes one (1-3
-// milliseconds), and gives it back. Two idle sets at most are kept per device,
+// Sets of chunks (1 MiB pinned, 8 MiB more once a set has copied 128 MiB),
+// streams and events are shared by the contexts of a process: a copy takes an
+// idle set of its device, or makes one (1-3 milliseconds), and gives it back. Two idle sets at most are kept per device,
 // and none once the device's last context is gone.
 
 // Every context holds one reference (stage_retain at its creation).

@@ -77,3 +77,26 @@ def test_forward_image_and_gradient_image(gpu):
         assert np.array_equal(img, film[..., :3] / film[..., 3:4])
     finally:
         r.close()
+
+
+def test_copies_after_a_set_has_taken_larger_chunks(gpu):
+    """1 MiB chunks from 128 MiB on: films around their ends and their rounds'."""
+    r = api.Renderer()
+    try:
+        r.upload(S.sunlit(64, 64, 1, 2))
+        r.render(1920, 1080, 1, 1)
+        for _ in range(4):  # 41 MB each
+            r.film(1920, 1080)
+        for mib in (1, 2, 4, 5, 8, 13):
+            for e in (-1, 0, 1):
+                w = -(-(mib << 20) // 20) + e
+                r.render(w, 1, 1, 1)
+                film = _locked((1, w, 5))
+                api.check(api.lib().ana_film_read(r.h, film.data_ptr(), w), r.h)
+                assert np.array_equal(film.numpy(), r.film(w, 1))
+        rays = random_rays(9 * (1 << 15) + 5, 11.0, 3)
+        locked, out = torch.from_numpy(rays).pin_memory(), _locked((len(rays), 8))
+        api.check(api.lib().ana_trace_batch(r.h, locked.data_ptr(), len(rays), out.data_ptr(), 0, 0), r.h)
+        assert out.numpy().tobytes() == r.trace(rays).tobytes()
+    finally:
+        r.close()

@@ -136,3 +136,28 @@ def test_a_copy_without_memory_for_its_threads(threads):
         rc = L.ana_film_read(r.h, out.ctypes.data, W * H)
         L.fake_fail_new(-1)
         assert rc == api.ANA_OK and np.array_equal(out, want)
+
+
+def test_sets_in_steady_use_take_larger_chunks():
+    """Once, after 128 MiB; without page-locked memory for them the small ones
+    stay in use, and are not given up."""
+    per = W * H * 20
+    reads = -(-(128 << 20) // per)
+    for refused in (False, True):
+        with fake_device() as L, closing(api.Renderer()) as r:
+            _rendered(r)
+            want = r.film(W, H)
+            made = L.fake_calls(b"cudaHostAlloc")
+            for _ in range(reads - 1):
+                r.film(W, H)
+            assert L.fake_calls(b"cudaHostAlloc") == made
+            waits = L.fake_calls(b"cudaEventSynchronize")
+            if refused:
+                L.fake_fail(b"cudaHostAlloc", 0, 1)
+            assert np.array_equal(r.film(W, H), want)
+            chunk = (1 << 17) if refused else (1 << 20)
+            assert L.fake_calls(b"cudaEventSynchronize") - waits == -(-per // chunk)
+            assert L.fake_calls(b"cudaHostAlloc") == made + 1
+            for _ in range(3):
+                assert np.array_equal(r.film(W, H), want)
+            assert L.fake_calls(b"cudaHostAlloc") == made + 1
