@@ -192,7 +192,7 @@ struct LevelArgs {
     const Open* open;      // this level's nodes
     Open* next;            // next level's nodes
     uint32_t* nextCount;
-    Open* small;           // subtrees left to one thread each
+    Open* small;           // subtrees left to one warp each
     uint32_t* smallCount;
     uint32_t nOpen;
     SlotInfo* info;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in,
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = tileSum[gridDim.x];
 }
 
-// ---- subtrees of at most kSmall triangles: one thread, sequential ----------
+// ---- subtrees of at most kSmall triangles: one warp each --------------------
 struct SmallArgs {
     Prims P;
     const Open* small;

@@ -128,8 +128,8 @@ void launch_film(const Params& p, const LaunchCfg& c, cudaStream_t s);
 // Adjoint replay stages: the shade / shadow / MIS kernels of the forward pass
 // with the gradient bookkeeping compiled in (identical sampling decisions),
 // the per-path delta set-up, and the resolution of the NEE and MIS gradient
-// payloads once their rays are traced.
-// Keeps a bounce's hits by path for the adjoint replay.
+// payloads once their rays are traced. launch_keep_hits, in the primal replay,
+// keeps a bounce's hits by path for the adjoint replay.
 void launch_keep_hits(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_adj_init(const Params& p, const LaunchCfg& c, cudaStream_t s);
 void launch_shade_adj(const Params& p, const LaunchCfg& c, cudaStream_t s);

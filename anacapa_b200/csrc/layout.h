@@ -1,7 +1,8 @@
 // Device-resident scene layout shared by the host preparation code and the
 // sm_100a kernels. Plain POD, no CUDA runtime calls.
 //
-// HBM layout (all arrays 16-byte aligned, read with 16-byte vector loads):
+// HBM layout (sections 256-byte aligned; nodes read with 32-byte vector loads,
+// the other records with 16-byte ones):
 //   tri_nodes   4-wide BVH nodes, 128 B each (Bvh4Node): the four children's
 //               boxes live in the parent so one node fetch tests four boxes.
 //   tri_isect   48 B per triangle in leaf order: (v0, orig index) (e1) (e2),

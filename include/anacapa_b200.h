@@ -300,7 +300,7 @@ int ana_upload_scene(ana_ctx* ctx, const ana_scene_desc* scene);
 
 /* ana_upload_scene with the triangle setup and SAH BVH build of
  * BVHBackend::commit (src/accel/BVHBackend.cpp:17-228) run on the device:
- * level-synchronous binned SAH over the large nodes, one thread per small
+ * level-synchronous binned SAH over the large nodes, one warp per small
  * subtree, the 4-wide collapse on the device. The uploaded bytes equal
  * ana_upload_scene's (ana_scene_digest). Curves, materials, lights and the
  * dome are prepared on the host as there. */
